@@ -1109,6 +1109,100 @@ __device__ __forceinline__ void block_run_chunk(const Csr<RP>& B, EnumSmem<NT>& 
   __syncthreads();
 }
 
+// Enumeration by groups: G = 2^lg lanes (at most a warp) walk one A entry's B
+// row, without the packing, the barriers and the owner search of the balanced
+// enumeration (banded 256/64, symbolic: 2.2 -> 1.9 ms). Rows whose B rows have
+// similar lengths and whose entries occupy the block's groups take it:
+// group_lanes returns lg when the padded steps (entries up to a multiple of
+// the groups, B rows up to a multiple of G) are at most three times the
+// products, and -1 otherwise. Long B rows (over 128 entries) stay with the
+// balanced enumeration, whose fast path walks them without a search and keeps
+// every warp busy on rows of one or two entries (power-law, symbolic hash_s:
+// 0.029 ms against 0.045 ms by groups).
+template <int NT>
+__device__ __forceinline__ int group_lanes(uint64_t anz, uint32_t np, uint32_t maxb) {
+  if (maxb > 128) return -1;
+  const int lg = maxb <= 4 ? 2 : min(5, 32 - __clz(maxb - 1));
+  const uint64_t pad = ((uint64_t)maxb + (1u << lg) - 1) >> lg << lg;
+  const uint64_t entries = (anz + (NT >> lg) - 1) / (NT >> lg) * (NT >> lg);
+  return entries * pad <= 3ull * np ? lg : -1;
+}
+
+// op(column, value) for every product of A entries [a0, a1), four entries per
+// group in flight. Not block-collective: the caller places the barriers.
+template <int NT, bool VALS, typename RP, typename Op>
+__device__ __forceinline__ void group_for_each_product(const Csr<RP>& A, const Csr<RP>& B, uint64_t a0, uint64_t a1,
+                                                       int lg, Op&& op) {
+  const uint32_t g = 1u << lg, sl = threadIdx.x & (g - 1), ng = NT >> lg;
+#pragma unroll 1
+  for (uint64_t k0 = a0 + (threadIdx.x >> lg); k0 < a1; k0 += 4 * ng) {
+    uint64_t b[4];
+    uint32_t len[4];
+    double av[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint64_t k = k0 + u * ng;
+      b[u] = 0;
+      len[u] = 0;
+      av[u] = 0.0;
+      if (k < a1) {
+        const uint32_t j = A.col[k];
+        b[u] = B.row_begin(j);
+        len[u] = (uint32_t)(B.row_end(j) - b[u]);
+        if (VALS) av[u] = A.val[k];
+      }
+    }
+    const uint32_t most = max(max(len[0], len[1]), max(len[2], len[3]));
+#pragma unroll 1
+    for (uint32_t t = sl; t < most; t += g) {
+      uint32_t c[4];
+      double bv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (t < len[u]) {
+          c[u] = B.col[b[u] + t];
+          if (VALS) bv[u] = B.val[b[u] + t];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t < len[u]) op(c[u], VALS ? av[u] * bv[u] : 0.0);
+    }
+  }
+}
+
+// The products of a row into registers, kUnroll per thread (c[u] = kEmpty:
+// none), by groups of 2^lg lanes with 2^lq steps per A entry; the row's
+// entries need at most kUnroll >> lq per group.
+template <int NT, typename RP>
+__device__ __forceinline__ void group_gather_once(const Csr<RP>& A, const Csr<RP>& B, uint64_t a0, uint64_t a1, int lg,
+                                                  int lq, uint32_t (&c)[kUnroll], double (&v)[kUnroll]) {
+  const uint32_t g = 1u << lg, sl = threadIdx.x & (g - 1), ng = NT >> lg;
+  uint64_t b[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const uint64_t k = a0 + (threadIdx.x >> lg) + (uint64_t)(u >> lq) * ng;
+    c[u] = kEmpty;
+    v[u] = 0.0;
+    b[u] = ~0ull;
+    if (k < a1) {
+      const uint32_t j = A.col[k];
+      const uint64_t at = B.row_begin(j) + (((uint32_t)u & ((1u << lq) - 1u)) << lg) + sl;
+      if (at < B.row_end(j)) {
+        b[u] = at;
+        v[u] = A.val[k];
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    if (b[u] != ~0ull) {
+      c[u] = B.col[b[u]];
+      v[u] *= B.val[b[u]];
+    }
+  }
+}
+
 // Enumerates every product of A entries [a0, a1) (all chunks).
 template <int NT, bool VALS, typename RP, typename Op>
 __device__ __forceinline__ void block_for_each_product(const Csr<RP>& A, const Csr<RP>& B, uint64_t a0,
@@ -1137,11 +1231,16 @@ __device__ __forceinline__ void mark_bit(unsigned long long* bits, uint32_t c, b
 }
 
 // ---------------------------------------------------------------- hash accumulators
-// Symbolic: one block per row, open-addressing set of column ids in shared memory
-// (linear probing, bounded by the table size).
+// Symbolic: one block per row. A row whose column span fits 32 columns per
+// table slot, with no more span words than products (so that clearing and
+// counting them does not dominate: power-law rows of 8192 products over 2^20
+// columns took 1.2 ms marked, 0.4 ms hashed), is marked in a bitmap laid over
+// the table, one test-before-set atomic per product; otherwise the columns go
+// to an open-addressing set in shared memory (linear probing, bounded by the
+// table size).
 template <int NT, int LOG2T>
 struct SymHashSmem {
-  uint32_t keys[1 << LOG2T];
+  uint32_t keys[1 << LOG2T];  // the set, or the span's bitmap
   EnumSmem<NT> e;
   unsigned long long red[33];
   uint32_t s_idx;
@@ -1149,13 +1248,13 @@ struct SymHashSmem {
 
 template <typename RP, int NT, int LOG2T>
 __global__ void __launch_bounds__(NT) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue q, DevCounters* __restrict__ ctr,
-                                                 const uint32_t* __restrict__ prod, const uint32_t* __restrict__ lo,
-                                                 const uint32_t* __restrict__ hi, uint32_t* __restrict__ row_nnz) {
-  constexpr int T = 1 << LOG2T;
+                                                 const uint32_t* __restrict__ prod, const uint32_t* __restrict__ maxb,
+                                                 const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
+                                                 uint32_t* __restrict__ row_nnz) {
+  constexpr uint32_t T = 1u << LOG2T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SymHashSmem<NT, LOG2T>& S = *reinterpret_cast<SymHashSmem<NT, LOG2T>*>(smem_raw);
   const int tid = threadIdx.x;
-  for (int i = tid; i < T; i += NT) S.keys[i] = kEmpty;
   const uint32_t count = *q.count;
   const uint32_t* list = q.rows;
   for (;;) {
@@ -1164,85 +1263,490 @@ __global__ void __launch_bounds__(NT) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue 
     const uint32_t idx = S.s_idx;
     if (idx >= count) break;
     const uint32_t row = list[idx];
-    // a row whose column span fits the table addresses it directly: slot = column - lo
     const uint32_t rlo = lo[row];
-    const bool direct = hi[row] - rlo < (uint32_t)T;
+    const uint32_t span1 = hi[row] - rlo;
+    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+    const uint32_t np = prod[row];
+    const int lg = group_lanes<NT>(a1 - a0, np, maxb[row]);
     unsigned cnt = 0;
-    bool full = false;
-    block_for_each_product<NT, false>(A, B, A.row_begin(row), A.row_end(row), S.e, [&](uint32_t c, double, bool ok) {
-      if (!ok) return;
-      uint32_t h = direct ? c - rlo : hash_slot(c, LOG2T);
-      int probe = 0;
-      for (; probe < T; ++probe) {
-        const uint32_t cur = S.keys[h];
-        if (cur == c) break;
-        if (cur == kEmpty) {
-          const uint32_t prev = atomicCAS(&S.keys[h], kEmpty, c);
-          if (prev == kEmpty) {
-            ++cnt;
-            break;
-          }
-          if (prev == c) break;
+    const uint32_t nw = (span1 >> 5) + 1;
+    if (nw <= T && nw <= np) {
+#pragma unroll 1
+      for (uint32_t i = tid; i < nw; i += NT) S.keys[i] = 0u;
+      auto mark = [&](uint32_t c) {
+        const uint32_t d = c - rlo;
+        if (d <= span1) {
+          const uint32_t m = 1u << (d & 31);
+          if (!(S.keys[d >> 5] & m)) atomicOr(&S.keys[d >> 5], m);
         }
-        h = (h + 1) & (T - 1);
+      };
+      if (lg >= 0) {
+        __syncthreads();
+        group_for_each_product<NT, false>(A, B, a0, a1, lg, [&](uint32_t c, double) { mark(c); });
+        __syncthreads();
+      } else {
+        // (block_load_chunk's barriers order the clearing before the marks)
+        block_for_each_product<NT, false>(A, B, a0, a1, S.e, [&](uint32_t c, double, bool ok) {
+          if (ok) mark(c);
+        });
       }
-      full |= probe == T;
-    });
-    if (full) raise_status(ctr, DEV_TABLE_FULL, row);
+#pragma unroll 1
+      for (uint32_t i = tid; i < nw; i += NT) cnt += __popc(S.keys[i]);
+    } else {
+      for (uint32_t i = tid; i < T; i += NT) S.keys[i] = kEmpty;
+      bool full = false;
+      auto insert = [&](uint32_t c) {
+        uint32_t h = hash_slot(c, LOG2T);
+        uint32_t probe = 0;
+#pragma unroll 1
+        for (; probe < T; ++probe) {
+          const uint32_t cur = S.keys[h];
+          if (cur == c) break;
+          if (cur == kEmpty) {
+            const uint32_t prev = atomicCAS(&S.keys[h], kEmpty, c);
+            if (prev == kEmpty) {
+              ++cnt;
+              break;
+            }
+            if (prev == c) break;
+          }
+          h = (h + 1) & (T - 1);
+        }
+        full |= probe == T;
+      };
+      if (lg >= 0) {
+        __syncthreads();
+        group_for_each_product<NT, false>(A, B, a0, a1, lg, [&](uint32_t c, double) { insert(c); });
+      } else {
+        block_for_each_product<NT, false>(A, B, a0, a1, S.e, [&](uint32_t c, double, bool ok) {
+          if (ok) insert(c);
+        });
+      }
+      if (full) raise_status(ctr, DEV_TABLE_FULL, row);
+    }
     const unsigned long long total = block_sum_u64<NT>(cnt, S.red);
     if (tid == 0) row_nnz[row] = (uint32_t)total;
-    for (int i = tid; i < T; i += NT) S.keys[i] = kEmpty;
   }
 }
 
-// Numeric: hash-accumulate FP64 values in shared memory, then write the row in
-// column order directly into C: rows whose span fits the table were addressed
-// directly and are compacted in slot order; the others are radix-sorted on
-// packed (column offset, dense index) words, or, when the span is too wide for
-// the packing, bitonic-sorted as (column << 32 | slot) keys.
+// Numeric kernel of the mid rows (classes hash_s/m/l): one block per row, FP64
+// sums in shared memory, the row written in column order straight into C
+// without a comparison sort. Three forms, by the row's column span and products:
+//  * dense (span <= 2 SLOTS): one slot per column; an occupancy bitmap gives
+//    each column its output position. One pass over the products.
+//  * bucket (at most kUnroll * NT products, kept in registers): the products
+//    are dealt into four buckets of equal column width per product slot (one
+//    shared atomic each), scattered to bucket order, and every product finds
+//    its rank and the products of its column among the one or two entries of
+//    its bucket. Rows so skewed that a bucket holds kBucketMax products take
+//    the next form.
+//  * rank: a two-level bitmap of the row's columns is built (level 1: which
+//    32-column words occur, level 2: the occurring words only, so the
+//    structures are as small as the row whatever its span); a product's slot
+//    is the rank of its column, two popcounts away.
+// Rows wider than 2^20 columns are left to k_num_hash. Against the hash table
+// with a radix sort that these rows took before (class kernel, one B200): 2^18
+// uniform rows of 32, bucket form, 13.1 -> 5.2 ms (3.2 GB of C; the gather of
+// the products is 2.0 ms of it, ordering them 1.9 ms, writing them 1.3 ms); 2 * 10^5
+// banded rows (256/64), dense form, 8.0 -> 4.4 ms (165 G products/s, bound by
+// the instructions of the enumeration and of the FP64 shared-memory sums); the
+// power-law 2^17 graph's rows of 512-2048 outputs 0.38 -> 0.20 ms. 64 registers
+// and 32 warps per SM; at 80 registers and 24 warps the bucket form is 10%
+// faster and the dense form 10% slower.
+constexpr uint32_t kBucketMax = 16;
+template <int NT, int SLOTS>
+struct NumRankSmem {
+  static constexpr int P = kUnroll * NT;  // products (and buckets) of a bucket row
+  union {
+    struct {
+      double vals[2 * SLOTS];
+      uint32_t bits[2 * SLOTS / 32];
+      uint32_t pre[2 * SLOTS / 32];
+    } d;
+    struct {
+      double vals[P];
+      uint32_t cols[P];
+      uint32_t cnt[P];         // products per bucket, four 8-bit counts a word
+      uint16_t pre[P];         // products of the buckets before each word
+      uint32_t lead[P / 32];   // slots that hold the first product of their column
+      uint32_t lpre[P / 32];   // such slots before each word
+    } b;
+    struct {
+      double vals[SLOTS];
+      uint32_t cols[SLOTS];
+      uint32_t wbits[SLOTS];               // level 2: the occurring 32-column words, in column order
+      uint16_t wpre[SLOTS];                // columns before each of them
+      uint32_t tbits[kBitmapBits / 1024];  // level 1: one bit per 32-column word
+      uint16_t tpre[kBitmapBits / 1024];   // occurring words before each level-1 word
+    } r;
+  };
+  EnumSmem<NT> e;
+  uint32_t s_idx, s_n, s_acc;
+};
+
+template <typename RP, int NT, int SLOTS>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B, RowQueue q, OutSpec o,
+                                                 DevCounters* __restrict__ ctr, const uint32_t* __restrict__ prod,
+                                                 const uint32_t* __restrict__ maxb, const uint32_t* __restrict__ lo,
+                                                 const uint32_t* __restrict__ hi, uint32_t* __restrict__ c_col,
+                                                 double* __restrict__ c_val) {
+  constexpr int NW = NT / 32;
+  constexpr int P = kUnroll * NT;
+  static_assert(kUnroll == 4, "one 16-byte group of bucket counts per thread");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  NumRankSmem<NT, SLOTS>& S = *reinterpret_cast<NumRankSmem<NT, SLOTS>*>(smem_raw);
+  uint32_t* const scan32 = reinterpret_cast<uint32_t*>(S.e.scan);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned lt = lanemask_lt();
+  const uint32_t count = *q.count;
+  const uint32_t* list = q.rows;
+  for (;;) {
+    if (tid == 0) S.s_idx = atomicAdd(q.cursor, 1u);
+    __syncthreads();
+    const uint32_t idx = S.s_idx;
+    if (idx >= count) break;
+    const uint32_t row = list[idx];
+    const uint32_t rlo = lo[row];
+    const uint32_t span1 = hi[row] - rlo;
+    const uint32_t np = prod[row];
+    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+    const uint32_t cap = o.cap[row];
+    const uint64_t off = o.off[row];
+    if (span1 >= (uint32_t)kBitmapBits) {  // k_num_hash's rows
+      __syncthreads();
+      continue;
+    }
+    const uint32_t mb = maxb[row];
+    const int lg = group_lanes<NT>(a1 - a0, np, mb);
+    if (span1 < 2u * SLOTS) {
+      const uint32_t nw = (span1 >> 5) + 1;
+#pragma unroll 1
+      for (uint32_t i = tid; i < nw; i += NT) S.d.bits[i] = 0u;
+#pragma unroll 1
+      for (uint32_t i = tid; i <= span1; i += NT) S.d.vals[i] = 0.0;
+      auto add = [&](uint32_t c, double v) {
+        const uint32_t d = c - rlo;
+        if (d <= span1) {
+          atomicAdd(&S.d.vals[d], v);
+          const uint32_t m = 1u << (d & 31);
+          if (!(S.d.bits[d >> 5] & m)) atomicOr(&S.d.bits[d >> 5], m);
+        }
+      };
+      if (lg >= 0) {
+        __syncthreads();
+        group_for_each_product<NT, true>(A, B, a0, a1, lg, add);
+        __syncthreads();
+      } else {
+        // (block_load_chunk's barriers order the clearing before the sums)
+        block_for_each_product<NT, true>(A, B, a0, a1, S.e, [&](uint32_t c, double v, bool ok) {
+          if (ok) add(c, v);
+        });
+      }
+      static_assert(2 * SLOTS / 32 <= NT, "one occupancy word per thread");
+      const uint32_t pc = (uint32_t)tid < nw ? __popc(S.d.bits[tid]) : 0u;
+      uint32_t n;
+      const uint32_t ex = block_excl_scan<NT, uint32_t>(pc, scan32, &n);
+      if ((uint32_t)tid < nw) S.d.pre[tid] = ex;
+      if (tid == 0) S.s_acc = out_accept(o, ctr, row, n, cap);
+      __syncthreads();
+      const uint32_t wn = S.s_acc ? min(n, cap) : 0u;
+#pragma unroll 1
+      for (uint32_t w = warp; w < nw; w += NW) {
+        const uint32_t bits = S.d.bits[w];
+        const uint32_t at = S.d.pre[w] + __popc(bits & lt);
+        if (((bits >> lane) & 1u) && at < wn) {
+          c_col[off + at] = rlo + w * 32u + lane;
+          c_val[off + at] = S.d.vals[w * 32u + lane];
+        }
+      }
+      __syncthreads();
+      continue;
+    }
+    // rows held in registers: gathered by groups, 2^lq steps per A entry
+    const int lq = lg < 0 || mb <= (1u << lg) ? 0 : (mb <= (2u << lg) ? 1 : 2);
+    const bool regs = lg >= 0 && np <= (uint32_t)P && mb <= (4u << lg) &&
+                      (((a1 - a0) + (NT >> lg) - 1) / (NT >> lg)) << lq <= (uint64_t)kUnroll;
+    uint32_t c[kUnroll], t[kUnroll];
+    double v[kUnroll];
+    if (regs) {
+      group_gather_once<NT>(A, B, a0, a1, lg, lq, c, v);
+      reinterpret_cast<uint4*>(S.b.cnt)[tid] = make_uint4(0u, 0u, 0u, 0u);
+      // bucket = column offset >> sh: at most 4 P buckets
+      constexpr int LOGP = NT == 128 ? 9 : (NT == 256 ? 10 : 11);
+      static_assert((1 << LOGP) == P, "bucket count");
+      const int sh = max(0, 32 - __clz(span1) - (LOGP + 2));
+      __syncthreads();
+      bool crowded = false;
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        t[u] = 0;
+        if (c[u] != kEmpty) {
+          c[u] -= rlo;
+          if (c[u] <= span1) {
+            const uint32_t bk = c[u] >> sh, s8 = (bk & 3u) * 8u;
+            t[u] = (atomicAdd(&S.b.cnt[bk >> 2], 1u << s8) >> s8) & 255u;
+            crowded |= t[u] >= kBucketMax;
+          } else {
+            c[u] = kEmpty;
+          }
+        }
+      }
+      if (!__syncthreads_or(crowded)) {
+        const uint4 k = reinterpret_cast<const uint4*>(S.b.cnt)[tid];
+        const uint32_t k0 = __dp4a(k.x, 0x01010101u, 0u), k1 = __dp4a(k.y, 0x01010101u, k0),
+                       k2 = __dp4a(k.z, 0x01010101u, k1), k3 = __dp4a(k.w, 0x01010101u, k2);
+        uint32_t total;
+        const uint32_t ex = block_excl_scan<NT, uint32_t>(k3, scan32, &total);
+        reinterpret_cast<uint2*>(S.b.pre)[tid] = make_uint2(ex | (ex + k0) << 16, (ex + k1) | (ex + k2) << 16);
+        __syncthreads();
+        // first slot of a bucket; n gets its products
+        auto bucket = [&](uint32_t d, uint32_t& n) {
+          const uint32_t bk = d >> sh, s8 = (bk & 3u) * 8u;
+          const uint32_t w = S.b.cnt[bk >> 2];
+          n = (w >> s8) & 255u;
+          return __dp4a(w & ((1u << s8) - 1u), 0x01010101u, (uint32_t)S.b.pre[bk >> 2]);
+        };
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+          if (c[u] != kEmpty) {
+            uint32_t len;
+            const uint32_t at = bucket(c[u], len) + t[u];
+            S.b.cols[at] = c[u];
+            S.b.vals[at] = v[u];
+          }
+        }
+        __syncthreads();
+        // slot by slot (each warp 32 consecutive ones): the first product of a
+        // column leads and takes the sum of the column's products
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+          const uint32_t i = (uint32_t)(u * NT + tid);
+          bool leads = false;
+          c[u] = kEmpty;
+          if (i < total) {
+            const uint32_t d = S.b.cols[i];
+            double sum = S.b.vals[i];
+            uint32_t len, smaller = 0;
+            const uint32_t s0 = bucket(d, len);
+            leads = true;
+            if (len > 1) {
+#pragma unroll 1
+              for (uint32_t j = s0; j < s0 + len; ++j) {
+                const uint32_t e = S.b.cols[j];
+                smaller += e < d;
+                if (e == d && j != i) {
+                  if (j < i) leads = false;
+                  else sum += S.b.vals[j];
+                }
+              }
+            }
+            c[u] = d;
+            // of two products a bucket's smaller one is a column of its own;
+            // of more, equal ones are told apart below by their leaders
+            t[u] = s0 | smaller << 16 | (len > 2 ? len << 24 : 0u);
+            v[u] = sum;
+          }
+          const unsigned m = __ballot_sync(kFull, leads);
+          if (lane == 0) S.b.lead[i >> 5] = m;
+          if (!leads) c[u] = kEmpty;
+        }
+        __syncthreads();
+        if (warp == 0) {
+          constexpr int WPL = (P / 32 + 31) / 32;
+          uint32_t x[WPL], sum = 0;
+#pragma unroll
+          for (int i = 0; i < WPL; ++i) {
+            const int w = lane * WPL + i;
+            x[i] = w < P / 32 ? __popc(S.b.lead[w]) : 0u;
+            sum += x[i];
+          }
+          uint32_t incl = sum;
+#pragma unroll
+          for (int sft = 1; sft < 32; sft <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, sft);
+            if (lane >= sft) incl += y;
+          }
+          uint32_t run = incl - sum;
+#pragma unroll
+          for (int i = 0; i < WPL; ++i) {
+            const int w = lane * WPL + i;
+            if (w < P / 32) S.b.lpre[w] = run;
+            run += x[i];
+          }
+          if (lane == 31) {
+            S.s_n = incl;
+            S.s_acc = out_accept(o, ctr, row, incl, cap);
+          }
+        }
+        __syncthreads();
+        const uint32_t wn = S.s_acc ? min(S.s_n, cap) : 0u;
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+          if (c[u] != kEmpty) {
+            const uint32_t s0 = t[u] & 0xFFFFu, len = t[u] >> 24;
+            uint32_t at = S.b.lpre[s0 >> 5] + __popc(S.b.lead[s0 >> 5] & ((1u << (s0 & 31)) - 1u));
+            if (len) {
+#pragma unroll 1
+              for (uint32_t j = s0; j < s0 + len; ++j)
+                at += S.b.cols[j] < c[u] && ((S.b.lead[j >> 5] >> (j & 31)) & 1u);
+            } else {
+              at += (t[u] >> 16) & 255u;
+            }
+            if (at < wn) {
+              c_col[off + at] = c[u] + rlo;
+              c_val[off + at] = v[u];
+            }
+          }
+        }
+        __syncthreads();
+        continue;
+      }
+    }
+    const uint32_t ntop = (span1 >> 10) + 1;
+    const uint32_t up = min(min(np, span1 + 1), (uint32_t)SLOTS);  // most entries (and words) the slots can hold
+    for (uint32_t i = tid; i < ntop; i += NT) S.r.tbits[i] = 0u;
+    for (uint32_t i = tid; i < up; i += NT) {
+      S.r.wbits[i] = 0u;
+      S.r.vals[i] = 0.0;
+    }
+    auto mark_top = [&](uint32_t d) {
+      const uint32_t m = 1u << ((d >> 5) & 31);
+      if (!(S.r.tbits[d >> 10] & m)) atomicOr(&S.r.tbits[d >> 10], m);
+    };
+    auto word_of = [&](uint32_t d) {
+      return (uint32_t)S.r.tpre[d >> 10] + __popc(S.r.tbits[d >> 10] & ((1u << ((d >> 5) & 31)) - 1u));
+    };
+    auto mark_word = [&](uint32_t w, uint32_t d) {
+      const uint32_t m = 1u << (d & 31);
+      if (!(S.r.wbits[w] & m)) atomicOr(&S.r.wbits[w], m);
+    };
+    auto accumulate = [&](uint32_t w, uint32_t d, double val) {
+      const uint32_t k = (uint32_t)S.r.wpre[w] + __popc(S.r.wbits[w] & ((1u << (d & 31)) - 1u));
+      S.r.cols[k] = d;
+      atomicAdd(&S.r.vals[k], val);
+    };
+    // exclusive popcounts of n words; returns their sum
+    auto scan_words = [&](const uint32_t* bits, uint16_t* pre, uint32_t n) {
+      const uint32_t per = ((n + NT - 1) / NT) | 1u;  // odd: the threads' strided reads touch all banks
+      const uint32_t i0 = min((uint32_t)tid * per, n), i1 = min(i0 + per, n);
+      uint32_t sum = 0;
+      for (uint32_t i = i0; i < i1; ++i) sum += __popc(bits[i]);
+      uint32_t total;
+      uint32_t run = block_excl_scan<NT, uint32_t>(sum, scan32, &total);
+      for (uint32_t i = i0; i < i1; ++i) {
+        pre[i] = (uint16_t)run;
+        run += __popc(bits[i]);
+      }
+      return total;
+    };
+    // op(column offset) for every product, then a barrier
+    auto each_col = [&](auto&& op) {
+      block_for_each_product<NT, false>(A, B, a0, a1, S.e, [&](uint32_t col, double, bool ok) {
+        if (ok && col - rlo <= span1) op(col - rlo);
+      });
+    };
+    // pass 1: the occurring words
+    if (regs) {
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u)
+        if (c[u] != kEmpty) mark_top(c[u]);
+      __syncthreads();
+    } else {
+      each_col([&](uint32_t d) { mark_top(d); });
+    }
+    const uint32_t nwords = scan_words(S.r.tbits, S.r.tpre, ntop);
+    __syncthreads();
+    uint32_t n = kUnknownCount;  // more words than slots: the row cannot be counted here
+    if (nwords <= (uint32_t)SLOTS) {
+      // pass 2: the occurring words' columns
+      if (regs) {
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u) {
+          if (c[u] != kEmpty) {
+            t[u] = word_of(c[u]);
+            mark_word(t[u], c[u]);
+          }
+        }
+        __syncthreads();
+      } else {
+        each_col([&](uint32_t d) { mark_word(word_of(d), d); });
+      }
+      n = scan_words(S.r.wbits, S.r.wpre, nwords);
+    }
+    if (tid == 0) {
+      if (!o.count && n > (uint32_t)SLOTS) raise_status(ctr, DEV_TABLE_FULL, row);
+      S.s_acc = out_accept(o, ctr, row, n, cap) && n <= (uint32_t)SLOTS;
+    }
+    __syncthreads();
+    if (S.s_acc) {
+      // pass 3: sums at the columns' ranks (n <= SLOTS, so every rank has a slot)
+      if (regs) {
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+          if (c[u] != kEmpty) accumulate(t[u], c[u], v[u]);
+        __syncthreads();
+      } else {
+        block_for_each_product<NT, true>(A, B, a0, a1, S.e, [&](uint32_t col, double val, bool ok) {
+          const uint32_t d = col - rlo;
+          if (ok && d <= span1) accumulate(word_of(d), d, val);
+        });
+      }
+      const uint32_t wn = min(n, cap);
+      for (uint32_t i = tid; i < wn; i += NT) {
+        c_col[off + i] = S.r.cols[i] + rlo;
+        c_val[off + i] = S.r.vals[i];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Rows of the hash classes whose span exceeds 2^20 columns: open addressing in
+// shared memory, then a radix sort of packed (column offset, dense index)
+// words, or, when the span is too wide for the packing, a bitonic sort of
+// (column << 32 | slot) keys. Launched only for B of more than 2^20 columns;
+// the blocks stride over the class list and leave the other rows to
+// k_num_rank.
 template <int NT, int LOG2T>
 struct NumHashSmem {
   double vals[1 << LOG2T];
   uint32_t keys[1 << LOG2T];  // reused as (1 << LOG2T) / 2 sort keys of 64 bits, or two radix buffers
   EnumSmem<NT> e;  // after the products: radix digit counts and dense-to-slot map
-  uint32_t s_idx, s_n, s_acc;
+  uint32_t s_n, s_acc;
 };
 
 template <typename RP, int NT, int LOG2T>
 __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue q, OutSpec o,
-                                                 DevCounters* __restrict__ ctr, const uint32_t* __restrict__ prod,
-                                                 const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
-                                                 uint32_t* __restrict__ c_col, double* __restrict__ c_val) {
+                                                 DevCounters* __restrict__ ctr, const uint32_t* __restrict__ lo,
+                                                 const uint32_t* __restrict__ hi, uint32_t* __restrict__ c_col,
+                                                 double* __restrict__ c_val) {
   constexpr int T = 1 << LOG2T;
   constexpr int PER = T / NT;
   constexpr int CAP = T / 2;  // sort capacity (entries) in the reused key area
+  constexpr int NW = NT / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   NumHashSmem<NT, LOG2T>& S = *reinterpret_cast<NumHashSmem<NT, LOG2T>*>(smem_raw);
-  unsigned long long* sortbuf = reinterpret_cast<unsigned long long*>(S.keys);
-  const int tid = threadIdx.x;
-  for (int i = tid; i < T; i += NT) {
-    S.keys[i] = kEmpty;
-    S.vals[i] = 0.0;
-  }
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t count = *q.count;
-  const uint32_t* list = q.rows;
-  for (;;) {
-    if (tid == 0) {
-      S.s_idx = atomicAdd(q.cursor, 1u);
-      S.s_n = 0;
-    }
-    __syncthreads();
-    const uint32_t idx = S.s_idx;
-    if (idx >= count) break;
-    const uint32_t row = list[idx];
-    // a row whose column span fits the table addresses it directly (slot =
-    // column - lo): no probing, and the slots are already in column order
+  for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
+    const uint32_t row = q.rows[idx];
     const uint32_t rlo = lo[row];
-    const bool direct = hi[row] - rlo < (uint32_t)T;
+    const uint32_t span1 = hi[row] - rlo;
+    if (span1 < (uint32_t)kBitmapBits) continue;
+    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+    const uint32_t cap = o.cap[row];
+    const uint64_t off = o.off[row];
+    if (tid == 0) S.s_n = 0;
+    unsigned long long* sortbuf = reinterpret_cast<unsigned long long*>(S.keys);
+    for (int i = tid; i < T; i += NT) {
+      S.keys[i] = kEmpty;
+      S.vals[i] = 0.0;
+    }
     bool full = false;
-    block_for_each_product<NT, true>(A, B, A.row_begin(row), A.row_end(row), S.e, [&](uint32_t c, double v, bool ok) {
+    block_for_each_product<NT, true>(A, B, a0, a1, S.e, [&](uint32_t c, double v, bool ok) {
       if (!ok) return;
-      uint32_t h = direct ? c - rlo : hash_slot(c, LOG2T);
+      uint32_t h = hash_slot(c, LOG2T);
       int probe = 0;
       for (; probe < T; ++probe) {
         const uint32_t cur = S.keys[h];
@@ -1265,51 +1769,16 @@ __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue 
     // with unknown count in estimation mode
     const int any_full = __syncthreads_or(full);
     if (any_full && tid == 0 && !o.count) raise_status(ctr, DEV_TABLE_FULL, row);
-    if (direct) {
-      // ordered compaction: thread t owns slots [t * PER, t * PER + PER); a
-      // block scan of the occupied counts gives each thread its output position
-      unsigned cnt = 0;
-#pragma unroll
-      for (int i = 0; i < PER; ++i) cnt += S.keys[tid * PER + i] != kEmpty;
-      unsigned long long n64;
-      const unsigned long long pos0 = block_excl_scan<NT, unsigned long long>(cnt, S.e.scan, &n64);
-      const uint32_t n = (uint32_t)n64;
-      const uint32_t cap = o.cap[row];
-      if (tid == 0) S.s_acc = out_accept(o, ctr, row, n, cap);
-      __syncthreads();
-      const uint32_t wn = S.s_acc ? min(n, cap) : 0u;
-      const uint64_t off = o.off[row];
-      uint32_t w = (uint32_t)pos0;
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const uint32_t sl = tid * PER + i;
-        const uint32_t key = S.keys[sl];
-        if (key != kEmpty) {
-          if (w < wn) {
-            c_col[off + w] = key;
-            c_val[off + w] = S.vals[sl];
-          }
-          ++w;
-          S.keys[sl] = kEmpty;
-          S.vals[sl] = 0.0;
-        }
-      }
-      __syncthreads();
-      continue;
-    }
-    // Rows whose span fits 32 - IB bits (the common case) are sorted by an LSD
+    // Rows whose span fits 32 - IB bits are sorted by an LSD
     // radix sort of one packed word per entry, (column - lo) << IB | dense
-    // index, 7 bits a pass (3 passes for a 2^20-column span, ~15 barriers
+    // index, 7 bits a pass (3-4 passes, 15-20 barriers
     // instead of the bitonic network's 78 for 4096 entries). The digit counts
     // and the dense-index-to-slot map live in the product enumerator's arrays,
     // free by now (8 NT + T bytes <= 24 NT bytes for every class); values
     // stay in their slots.
     constexpr int IB = LOG2T - 1;  // bits of a dense index below CAP = T / 2
-    constexpr int NW = NT / 32;
     constexpr int RB = 128;        // buckets of a 7-bit digit
     static_assert(2 * RB * NW + 2 * CAP <= (int)(3 * sizeof(unsigned long long) * NT), "radix scratch");
-    const int warp = tid >> 5, lane = tid & 31;
-    const uint32_t span1 = hi[row] - rlo;
     if (!any_full && span1 < (1u << (32 - IB))) {
       uint16_t* hist = reinterpret_cast<uint16_t*>(S.e.incl);  // [RB][NW]
       uint16_t* dslot = hist + RB * NW;                         // [CAP]
@@ -1390,7 +1859,6 @@ __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue 
           kout = t;
         }
       }
-      const uint32_t cap = o.cap[row];
       if (tid == 0) {
         const bool acc = out_accept(o, ctr, row, n, cap);
         if (!o.count && n > CAP) raise_status(ctr, DEV_COUNT_MISMATCH, row);
@@ -1398,17 +1866,12 @@ __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue 
       }
       __syncthreads();
       const uint32_t wn = S.s_acc ? min(n, cap) : 0u;
-      const uint64_t off = o.off[row];
       for (uint32_t i = tid; i < wn; i += NT) {
         const uint32_t key = kin[i];
         c_col[off + i] = (key >> IB) + rlo;
         c_val[off + i] = S.vals[dslot[key & ((1u << IB) - 1u)]];
       }
       __syncthreads();
-      for (int i = tid; i < T; i += NT) {
-        S.keys[i] = kEmpty;
-        S.vals[i] = 0.0;
-      }
       continue;
     }
     // compaction: read this thread's slots, then rewrite the key area as sort keys
@@ -1451,7 +1914,6 @@ __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue 
         __syncthreads();
       }
     }
-    const uint32_t cap = o.cap[row];
     if (tid == 0) {
       const uint32_t nn = any_full ? kUnknownCount : n;
       bool acc = out_accept(o, ctr, row, nn, cap);
@@ -1461,17 +1923,12 @@ __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue 
     __syncthreads();
     // rows that overflowed the sort capacity or their slots are not written
     const uint32_t wn = S.s_acc ? min(n, cap) : 0u;
-    const uint64_t off = o.off[row];
     for (uint32_t i = tid; i < wn; i += NT) {
       const unsigned long long e = sortbuf[i];
       c_col[off + i] = (uint32_t)(e >> 32);
       c_val[off + i] = S.vals[(uint32_t)e];
     }
     __syncthreads();
-    for (int i = tid; i < T; i += NT) {
-      S.keys[i] = kEmpty;
-      S.vals[i] = 0.0;
-    }
   }
 }
 
@@ -2514,6 +2971,8 @@ constexpr size_t kWinNumSmem = sizeof(WinNumSmem);
 constexpr size_t kSymBitmapSmem = sizeof(BitmapSymSmem);
 template <int NT, int LOG2T>
 constexpr size_t num_hash_smem() { return sizeof(NumHashSmem<NT, LOG2T>); }
+template <int NT, int SLOTS>
+constexpr size_t num_rank_smem() { return sizeof(NumRankSmem<NT, SLOTS>); }
 template <int NT, int LOG2T>
 constexpr size_t sym_hash_smem() { return sizeof(SymHashSmem<NT, LOG2T>); }
 
@@ -2543,8 +3002,11 @@ void set_attrs() {
   allow_smem(k_sym_hash<RP, 256, 13>, sym_hash_smem<256, 13>());
   allow_smem(k_sym_hash<RP, 512, 15>, sym_hash_smem<512, 15>());
   allow_smem(k_num_hash<RP, 128, 10>, num_hash_smem<128, 10>());
+  allow_smem(k_num_rank<RP, 128, 512>, num_rank_smem<128, 512>());
   allow_smem(k_num_hash<RP, 256, 12>, num_hash_smem<256, 12>());
+  allow_smem(k_num_rank<RP, 256, 2048>, num_rank_smem<256, 2048>());
   allow_smem(k_num_hash<RP, 512, 13>, num_hash_smem<512, 13>());
+  allow_smem(k_num_rank<RP, 512, 4096>, num_rank_smem<512, 4096>());
 }
 }  // namespace
 
@@ -2561,9 +3023,9 @@ void configure_kernel_attributes() {
   g_occ[K_NUM_ESC1] = occ_of(k_num_esc<uint32_t, 1>, 256, 0);
   g_occ[K_NUM_ESC2] = occ_of(k_num_esc<uint32_t, 2>, 256, 0);
   g_occ[K_NUM_ESC4] = occ_of(k_num_esc<uint32_t, 4>, 256, 0);
-  g_occ[K_NUM_S] = occ_of(k_num_hash<uint32_t, 128, 10>, 128, num_hash_smem<128, 10>());
-  g_occ[K_NUM_M] = occ_of(k_num_hash<uint32_t, 256, 12>, 256, num_hash_smem<256, 12>());
-  g_occ[K_NUM_L] = occ_of(k_num_hash<uint32_t, 512, 13>, 512, num_hash_smem<512, 13>());
+  g_occ[K_NUM_S] = occ_of(k_num_rank<uint32_t, 128, 512>, 128, num_rank_smem<128, 512>());
+  g_occ[K_NUM_M] = occ_of(k_num_rank<uint32_t, 256, 2048>, 256, num_rank_smem<256, 2048>());
+  g_occ[K_NUM_L] = occ_of(k_num_rank<uint32_t, 512, 4096>, 512, num_rank_smem<512, 4096>());
   g_occ[K_NUM_BM] = occ_of(k_num_bitmap<uint32_t>, kBitmapThreads, kNumBitmapSmem);
   g_occ[K_NUM_WIN] = occ_of(k_num_window<uint32_t>, kBitmapThreads, kWinNumSmem);
 }
@@ -2661,15 +3123,15 @@ int launch_symbolic(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, int nu
     k_sym_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(SB_ESC4), w.ctr, w.row_nnz);
   mark(SB_HASH_S);
   if ((gsz = grid(K_SYM_S, SB_HASH_S, 1)) && ++launched)
-    k_sym_hash<RP, 128, 11><<<gsz, 128, sym_hash_smem<128, 11>(), s>>>(A, B, queue(SB_HASH_S), w.ctr, w.prod,
+    k_sym_hash<RP, 128, 11><<<gsz, 128, sym_hash_smem<128, 11>(), s>>>(A, B, queue(SB_HASH_S), w.ctr, w.prod, w.maxb,
                                                                        w.lo, w.hi, w.row_nnz);
   mark(SB_HASH_M);
   if ((gsz = grid(K_SYM_M, SB_HASH_M, 1)) && ++launched)
-    k_sym_hash<RP, 256, 13><<<gsz, 256, sym_hash_smem<256, 13>(), s>>>(A, B, queue(SB_HASH_M), w.ctr, w.prod,
+    k_sym_hash<RP, 256, 13><<<gsz, 256, sym_hash_smem<256, 13>(), s>>>(A, B, queue(SB_HASH_M), w.ctr, w.prod, w.maxb,
                                                                        w.lo, w.hi, w.row_nnz);
   mark(SB_HASH_L);
   if ((gsz = grid(K_SYM_L, SB_HASH_L, 1)) && ++launched)
-    k_sym_hash<RP, 512, 15><<<gsz, 512, sym_hash_smem<512, 15>(), s>>>(A, B, queue(SB_HASH_L), w.ctr, w.prod,
+    k_sym_hash<RP, 512, 15><<<gsz, 512, sym_hash_smem<512, 15>(), s>>>(A, B, queue(SB_HASH_L), w.ctr, w.prod, w.maxb,
                                                                        w.lo, w.hi, w.row_nnz);
   mark(SB_BITMAP);
   if ((gsz = grid(K_SYM_BM, SB_BITMAP, 1)) && ++launched)
@@ -2743,6 +3205,7 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
     return RowQueue{w.num_bins + (uint64_t)c * A.rows, w.ctr->num_count + c, w.ctr->num_cursor + c};
   };
   unsigned gsz;
+  const bool wide = B.cols > kBitmapBits;  // only then can a row's span exceed 2^20 columns
   mark(NB_ESC1);
   if ((gsz = grid(K_NUM_ESC1, NB_ESC1, 8)) && ++launched)
     k_num_esc<RP, 1><<<gsz, 256, 0, s>>>(A, B, queue(NB_ESC1), o, w.ctr, c_col, c_val);
@@ -2754,16 +3217,25 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
     k_num_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(NB_ESC4), o, w.ctr, c_col, c_val);
   mark(NB_HASH_S);
   if ((gsz = grid(K_NUM_S, NB_HASH_S, 1)) && ++launched)
-    k_num_hash<RP, 128, 10><<<gsz, 128, num_hash_smem<128, 10>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.prod,
-                                                                       w.lo, w.hi, c_col, c_val);
+    k_num_rank<RP, 128, 512><<<gsz, 128, num_rank_smem<128, 512>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.prod, w.maxb,
+                                                                  w.lo, w.hi, c_col, c_val);
+  if (wide && gsz && ++launched)
+    k_num_hash<RP, 128, 10><<<gsz, 128, num_hash_smem<128, 10>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.lo, w.hi,
+                                                                  c_col, c_val);
   mark(NB_HASH_M);
   if ((gsz = grid(K_NUM_M, NB_HASH_M, 1)) && ++launched)
-    k_num_hash<RP, 256, 12><<<gsz, 256, num_hash_smem<256, 12>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.prod,
-                                                                       w.lo, w.hi, c_col, c_val);
+    k_num_rank<RP, 256, 2048><<<gsz, 256, num_rank_smem<256, 2048>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.prod, w.maxb,
+                                                                  w.lo, w.hi, c_col, c_val);
+  if (wide && gsz && ++launched)
+    k_num_hash<RP, 256, 12><<<gsz, 256, num_hash_smem<256, 12>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.lo, w.hi,
+                                                                  c_col, c_val);
   mark(NB_HASH_L);
   if ((gsz = grid(K_NUM_L, NB_HASH_L, 1)) && ++launched)
-    k_num_hash<RP, 512, 13><<<gsz, 512, num_hash_smem<512, 13>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.prod,
-                                                                       w.lo, w.hi, c_col, c_val);
+    k_num_rank<RP, 512, 4096><<<gsz, 512, num_rank_smem<512, 4096>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.prod, w.maxb,
+                                                                  w.lo, w.hi, c_col, c_val);
+  if (wide && gsz && ++launched)
+    k_num_hash<RP, 512, 13><<<gsz, 512, num_hash_smem<512, 13>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.lo, w.hi,
+                                                                  c_col, c_val);
   mark(NB_BITMAP);
   const bool windowed = !o.count && w.win_cursor && w.win_scratch;
   if (windowed) {

@@ -1,0 +1,125 @@
+"""Forms of the mid-row kernels (dense, bucket, rank, hash by span; marked or
+hashed symbolic rows): rows at the edges where one form gives way to the next,
+against the oracle. Structure bit for bit, values within 1e-12 of
+sum |a_ik * b_kj| (FP64 sums of at most 4096 terms in another order: below
+4096 * 2^-53 = 4.6e-13 of it)."""
+import numpy as np
+import pytest
+
+from research_b200 import matrices as M
+
+from test_gpu_parity import NUM_BINS, SYM_BINS, check, multiply_device
+
+pytestmark = pytest.mark.gpu
+
+CLASSES = {"hash_s": (128, 512), "hash_m": (256, 2048), "hash_l": (512, 4096)}  # threads, output entries
+
+
+def _product(span, entries, length, repeat, seed, skew=False):
+    """(A, B): B rows of `length` columns over exactly `span` columns, two in
+    `repeat` of them shared by several rows; A rows take `entries` of B's rows, one
+    fewer, and a third of them. skew: most columns are among the first 4096."""
+    rng = np.random.default_rng(seed)
+    rows, cols = [], []
+    pool = rng.choice(min(span, 4096) if skew else span, min(span, entries * length) if not skew else min(span, 4096),
+                      replace=False)
+    at = 0
+    for i in range(entries):
+        c = set()
+        while len(c) < min(length, span):
+            if repeat and len(c) < length // 2 and rng.random() < 2.0 / repeat:
+                c.add(int(pool[rng.integers(0, min(64, pool.size))]))
+            else:
+                c.add(int(pool[at % pool.size]) if at < 2 * pool.size else int(rng.integers(0, span)))
+                at += 1
+        c = sorted(c)
+        if i == 0:
+            c[0], c[-1] = 0, span - 1
+            c = sorted(set(c))
+        rows += [i] * len(c)
+        cols += c
+    B = M.from_coo(entries, span + 3, rows, cols, rng.uniform(-1, 1, len(rows)))
+    ar, ac = [], []
+    for r, k in enumerate((entries, max(1, entries - 1), max(1, entries // 3))):
+        ar += [r] * k
+        ac += list(range(k))
+    return M.from_coo(3, entries, ar, ac, rng.uniform(-1, 1, len(ar))), B
+
+
+def _run(A, B, num, sym="bitmap", **cfg):
+    C, _ = multiply_device(A, B, {"force_sym_bin": SYM_BINS[sym], "force_num_bin": NUM_BINS[num], **cfg})
+    check(A, B, C)
+
+
+@pytest.mark.parametrize("num", list(CLASSES))
+@pytest.mark.parametrize("edge", [-1, 0, 1])
+def test_products_at_the_register_limit(num, edge):
+    # 4 products per thread: one B row less, exactly, one more
+    threads, _ = CLASSES[num]
+    for length, repeat in ((32, 8), (16, 3), (5, 4)):
+        k = 4 * threads // length + edge
+        A, B = _product(200000, k, length, repeat, 10 * k + length)
+        if num == "hash_s" and np.unique(B.col).size > 512:
+            A, B = _product(200000, min(k, 500 // length), length, repeat, 3)
+        _run(A, B, num)
+
+
+@pytest.mark.parametrize("span", [1, 2, 33, 1023, 1024, 1025, 4096, 4097, 8192, 8193, 65536, (1 << 20) - 1, 1 << 20,
+                                  (1 << 20) + 1, 3 << 20])
+@pytest.mark.parametrize("num", list(CLASSES))
+def test_spans(num, span):
+    _, cap = CLASSES[num]
+    for entries, length in ((7, 60), (cap // 40, 37)):
+        A, B = _product(span, entries, min(length, span), 5, span % 1000 + entries)
+        _run(A, B, num)
+
+
+@pytest.mark.parametrize("num", list(CLASSES))
+def test_rows_that_fill_every_slot(num):
+    # as many distinct columns as the class holds, every column once
+    _, cap = CLASSES[num]
+    rng = np.random.default_rng(cap)
+    for span in (50000, 1 << 20):
+        cols = np.sort(rng.choice(span, cap, replace=False))
+        cols[0], cols[-1] = 0, span - 1
+        order = np.argsort(rng.random(cap)) % 16
+        B = M.from_coo(16, span, order, cols, rng.uniform(-1, 1, cap))
+        A = M.from_coo(1, 16, np.zeros(16, int), np.arange(16), rng.uniform(-1, 1, 16))
+        _run(A, B, num)
+
+
+@pytest.mark.parametrize("num", list(CLASSES))
+def test_skewed_columns_leave_the_bucket_form(num):
+    # most products in a few buckets, and one column shared by every B row
+    threads, _ = CLASSES[num]
+    A, B = _product(1 << 19, 3 * threads // 32, 32, 2, 77, skew=True)
+    _run(A, B, num)
+
+
+@pytest.mark.parametrize("wf", [1, 2])
+def test_forms_in_the_estimated_workflows(wf):
+    # sizes estimated: rows that outgrow their slots go through the overflow list
+    A = M.uniform_random(30000, 24, seed=4)
+    C, st = multiply_device(A, A, {"force_workflow": wf, "estimate_scale": 0.4})
+    check(A, A, C)
+    assert st["decision"]["workflow"] == wf
+
+
+@pytest.mark.parametrize("sym", list(CLASSES))
+@pytest.mark.parametrize("words", [15, 16, 17])
+def test_symbolic_marked_or_hashed(sym, words):
+    # span words just below, at and above the products: marked or hashed
+    A, B = _product(32 * 16 * words, 16, 16, 4, words)
+    _run(A, B, "bitmap", sym)
+
+
+def test_uneven_b_rows_take_the_balanced_enumeration():
+    rng = np.random.default_rng(5)
+    lens = np.r_[np.full(200, 2), 700, 300]
+    r = np.repeat(np.arange(lens.size), lens)
+    B = M.from_coo(lens.size, 90000, r, rng.integers(0, 90000, r.size), rng.uniform(-1, 1, r.size))
+    A = M.from_coo(2, lens.size, np.repeat([0, 1], lens.size), np.tile(np.arange(lens.size), 2),
+                   rng.uniform(-1, 1, 2 * lens.size))
+    for num in ("hash_m", "hash_l"):
+        for sym in CLASSES:
+            _run(A, B, num, sym if sym != "hash_s" else "hash_m")
