@@ -511,8 +511,12 @@ void make_segment_policies(const Config& c, const SymPolicy& sp, const NumPolicy
 const SymPolicy* seg_sym(const ocean_handle* h) { return h->seg_dispatch ? h->seg_sp : nullptr; }
 const NumPolicy* seg_num(const ocean_handle* h) { return h->seg_dispatch ? h->seg_np : nullptr; }
 
-// Phase 1: row analysis. Large inputs read the counters back (class sizes,
-// product totals); small inputs skip the read-back. Returns whether it read back.
+// Phase 1: row analysis. The counters (class sizes, product totals) are read
+// back, so that only the classes that have rows are launched: for a small
+// input one read-back (about 10 us) costs less than the launches of five
+// empty symbolic kernels (6-10 us each at full grid), and the bitmap rows of a
+// small A times a large B can save their bitmaps. Returns whether the input is
+// large enough (small_problem_nnz) for the workflow choice to look at them.
 template <typename RP>
 bool run_analysis(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s) {
   h->ev_recorded = false;  // the stats describe a completed multiply only
@@ -532,21 +536,18 @@ bool run_analysis(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
   h->st.launches = launch_analysis(A, B, h->w, sp, s);
   OCEAN_CUDA(cudaGetLastError());
   if (h->cfg.track_stage_times) record(h, EV_ANALYSIS, s);
-  const bool readback = A.nnz > (uint64_t)h->cfg.small_problem_nnz;
-  if (readback) {
-    OCEAN_CUDA(cudaMemcpyAsync(h->h_ctr, h->w.ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-    OCEAN_CUDA(wait_stream(s, h->cfg.spin_wait_us));
-  }
-  return readback;
+  OCEAN_CUDA(cudaMemcpyAsync(h->h_ctr, h->w.ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
+  OCEAN_CUDA(wait_stream(s, h->cfg.spin_wait_us));
+  return A.nnz > (uint64_t)h->cfg.small_problem_nnz;
 }
 
 // Segment-driven dispatch: the segments' row bands become per-row policy
 // slots (slot 1 + SegClass; a row inside several bands takes the first band
 // listed; rows in no band keep slot 0, the call's policy); then the analysis
-// classes every row again under its slot's policy and, for inputs that read
-// back, the counters are read back again.
+// classes every row again under its slot's policy and the counters are read
+// back again.
 template <typename RP>
-void dispatch_segments(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool readback) {
+void dispatch_segments(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s) {
   SymPolicy sp;
   NumPolicy np;
   make_policies(h->cfg, &sp, &np);
@@ -600,10 +601,8 @@ void dispatch_segments(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cuda
   OCEAN_CUDA(cudaMemsetAsync(h->w.ctr, 0, sizeof(DevCounters), s));
   h->st.launches += (n ? 1 : 0) + launch_analysis(A, B, h->w, sp, s, h->seg_sp);
   OCEAN_CUDA(cudaGetLastError());
-  if (readback) {
-    OCEAN_CUDA(cudaMemcpyAsync(h->h_ctr, h->w.ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-    OCEAN_CUDA(wait_stream(s, h->cfg.spin_wait_us));
-  }
+  OCEAN_CUDA(cudaMemcpyAsync(h->h_ctr, h->w.ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
+  OCEAN_CUDA(wait_stream(s, h->cfg.spin_wait_us));
 }
 
 // Buffers of the windowed exact numeric kernel for the bitmap class: cursors
@@ -640,28 +639,38 @@ void prepare_windows(ocean_handle* h, uint64_t a_nnz, unsigned bitmap_rows) {
 
 // Phase 2 of the precise workflow: symbolic class kernels (exact counts into
 // w.row_nnz) and, with_scan, the row-pointer scan and numeric class lists; the
-// counters are read back at the end. With allow_cache (and the class sizes of
-// a read-back), bitmap-class rows save their bitmaps into h->w.bm_cache, whose
-// size comes from the analysis and is capped by bitmap_cache_fraction of free memory.
+// counters are read back at the end. With allow_cache, bitmap-class rows save
+// their bitmaps into h->w.bm_cache, whose size comes from the analysis and is capped by bitmap_cache_fraction of free memory.
 template <typename RP>
-void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool readback,
-                  bool with_scan, bool allow_cache) {
+void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool with_scan,
+                  bool allow_cache) {
   SymPolicy sp;
   NumPolicy np;
   make_policies(h->cfg, &sp, &np);
   unsigned sym_counts[SB_COUNT];
   for (int i = 0; i < SB_COUNT; ++i) sym_counts[i] = h->h_ctr->sym_count[i];
-  if (readback && allow_cache && h->cfg.bitmap_cache_fraction > 0.0) {
+  if (allow_cache && h->cfg.bitmap_cache_fraction > 0.0) {
     const uint64_t want = h->h_ctr->sym_words;
-    const uint64_t budget =
-        want >= 1024 ? (uint64_t)(h->cfg.bitmap_cache_fraction * (double)available_device_bytes(h->device)) / 8 : 0;
+    // The free-memory query stalls the host for up to 10 ms when large results
+    // were just freed (power-law 2^17, the previous C still pending: 28 ms per
+    // multiply with it, 16 ms without): it is left out when the buffer of an
+    // earlier call is large enough, or when the bitmaps would fit their share
+    // of 4% of the device (an allocation that fails only turns the cache off).
+    const double share = h->cfg.bitmap_cache_fraction;
+    uint64_t budget = 0;
+    if (want >= 1024) {
+      if ((h->cache_buf && h->cache_cap_words >= want) || 8.0 * (double)want <= share * 0.04 * (double)h->device_bytes)
+        budget = want;
+      else
+        budget = (uint64_t)(share * (double)available_device_bytes(h->device)) / 8;
+    }
     const uint64_t words = std::min(want, budget);
     if (words >= 1024) {
       if (h->cache_cap_words < words) {
         if (h->cache_buf) cudaFree(h->cache_buf);
         h->cache_buf = nullptr;
         h->cache_cap_words = 0;
-        const uint64_t grow_to = std::min(budget, words + words / 8);
+        const uint64_t grow_to = std::max(words, std::min(budget, words + words / 8));
         if (cudaMalloc((void**)&h->cache_buf, grow_to * 8) == cudaSuccess) {
           h->cache_cap_words = grow_to;
         } else {
@@ -677,7 +686,7 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
   // per-class boundary events only when stage timing is asked for (each record costs device time)
   const bool track = h->cfg.track_stage_times;
   h->st.launches += launch_symbolic(A, B, h->w, h->num_sms, s, track ? h->ev + EV_SYM0 : nullptr,
-                                    readback ? sym_counts : nullptr);
+                                    sym_counts);
   if (track && A.rows) h->ev_mask |= ((1ull << (SB_COUNT + 1)) - 1) << EV_SYM0;
   OCEAN_CUDA(cudaGetLastError());
   if (with_scan) {
@@ -695,8 +704,8 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
 template <typename RP>
 void run_front(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool with_scan,
                bool allow_cache) {
-  const bool readback = run_analysis(h, A, B, s);
-  run_symbolic(h, A, B, s, readback, with_scan, allow_cache);
+  run_analysis(h, A, B, s);
+  run_symbolic(h, A, B, s, with_scan, allow_cache);
 }
 
 // Stops using the saved bitmaps for this call (the buffer stays with the handle).
@@ -1008,7 +1017,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
           // segment-driven dispatch (the reference's listed follow-up,
           // kernels/SpGEMM.cuh:241-244): every row of a segment takes its
           // class's policy, and the rows are classed again with them
-          dispatch_segments(h, A, B, s, readback);
+          dispatch_segments(h, A, B, s);
           mark("segment_dispatch");
         }
       }
@@ -1019,22 +1028,13 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
       bool class_counts = true;
       // ultra-sparse rows of at most 256 products: one fused launch writes C
       // in place (capacity: the product count, read back by the analysis).
-      // Small inputs skip the analysis read-back on the precise path; here
-      // the counters are read back once to see whether the fused path applies.
       const Config& cf = h->cfg;
       const bool fusable_cfg = cf.fused_ultrasparse && !cf.estimator_metrics && !cf.use_segment_dispatch &&
                                (cf.force_workflow == WF_ULTRASPARSE ||
                                 (cf.force_workflow < 0 && cf.use_ultrasparse_workflow));
-      bool fresh = readback;  // h_ctr holds this call's analysis counters
-      if (!readback && fusable_cfg && (wf == WF_PRECISE || wf == WF_ULTRASPARSE)) {
-        OCEAN_CUDA(cudaMemcpyAsync(h->h_ctr, h->w.ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-        OCEAN_CUDA(wait_stream(s, h->cfg.spin_wait_us));
-        fresh = true;
-        mark("fused_probe");
-      }
       const DevCounters& kc = *h->h_ctr;
-      const bool fits = fresh && kc.max_products <= kUspMaxProducts && kc.total_products < (1ull << 32);
-      if (fits && wf == WF_PRECISE && !readback && cf.force_workflow < 0 &&
+      const bool fits = kc.max_products <= kUspMaxProducts && kc.total_products < (1ull << 32);
+      if (fits && fusable_cfg && wf == WF_PRECISE && !readback && cf.force_workflow < 0 &&
           (double)kc.total_products <= cf.usparse_avg_product_threshold * (double)A.rows)
         wf = WF_ULTRASPARSE;
       st.fused = fits && fusable_cfg && wf == WF_ULTRASPARSE;
@@ -1088,7 +1088,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
       }
       if (st.fused) {
       } else if (wf == WF_PRECISE) {
-        run_symbolic(h, A, B, s, readback, true, true);
+        run_symbolic(h, A, B, s, true, true);
         mark("symbolic");
         nnz = h->h_ctr->total_nnz;
         if (h->w.chunks) {
