@@ -38,6 +38,13 @@ struct DevWork {
   uint32_t* win_cursor = nullptr;
   unsigned long long* win_scratch = nullptr;
   uint32_t wide_rows = 0xFFFFFFFFu;
+  // exact-mode numeric bitmap class: list of window items of the rows with a
+  // saved bitmap (capacity item_capacity), list of the other rows, and their
+  // counters; null items: every row runs whole in k_num_bitmap
+  void* items = nullptr;
+  uint32_t item_cap = 0;
+  uint32_t* item_rest = nullptr;
+  ItemCounters* item_ctr = nullptr;
   // rows of A with more than kLongRowEntries entries: listed by the analysis
   // and summarised (and HLL-merged) by all warps together; null: each row is
   // handled by its own lane group
@@ -203,6 +210,11 @@ int launch_row_bounds(const DevWork& w, uint32_t* out, cudaStream_t s);
 // every entry point that may be first on a device; false: bad ordinal).
 void configure_kernel_attributes();
 bool ensure_kernel_attributes(int dev);
+
+// Most window items of `rows` bitmap-class rows with `nnz` output entries, and
+// the bytes of one.
+uint64_t item_capacity(uint64_t rows, uint64_t nnz);
+size_t item_bytes();
 
 // Words of DevWork::win_scratch for a device with num_sms SMs (one 2^20-bit
 // bitmap per resident block of k_num_window); valid after configure_kernel_attributes.

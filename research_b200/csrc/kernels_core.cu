@@ -2495,6 +2495,344 @@ __global__ void __launch_bounds__(kBitmapThreads, 1)
   }
 }
 
+// ---------------------------------------------------------------- window items
+// Numeric kernel of bitmap-class rows whose bitmap the symbolic pass saved.
+// A row's output is cut into windows of whole 2048-column groups with at most
+// kItemV entries and kItemGroups groups (k_item_plan), and every window is a
+// work item of its own: the block loads the window's bitmap words and their
+// ranks into shared memory, finds the part of every referenced B row that lies
+// in the window by a search, sums the products in FP64 slots at the rank of
+// their column, and writes the window's columns and values once, in order. No
+// zero fill, no global atomic, and no row is too heavy for one block.
+// An item costs 15-22 thousand cycles for its products (0.9 per cycle and SM,
+// the FP64 shared-memory sums) and, on one block per SM, about as many for the
+// loads and searches before them, which grow with the span and the B rows.
+// So it takes (times of the numeric bitmap class on one B200, before -> after)
+//  * rows of at most kItemWideWords words of span: power-law 2^17 graph,
+//    11.6 -> 9.3 ms;
+//  * of wider rows, those with more products than a quarter of an SM's
+//    share of the class, which would otherwise run on in one block when all
+//    others are done: 1/32 of the rows of the power-law 2^20 graph times the
+//    graph, 13.3 -> 8.6 ms.
+// All rows of the 2^20 graph as items: 255 ms against 217 ms in k_num_bitmap.
+constexpr int kItemV = 10240;      // output entries per item (FP64 slots and columns in shared memory)
+constexpr int kItemGroups = 256;   // groups of 32 words (2048 columns) per item
+constexpr int kItemWords = kItemGroups * 32;
+constexpr uint32_t kItemWideWords = 4096;  // 2^18 columns
+
+struct WinItem {
+  uint32_t row, g0, g1;  // groups [g0, g1) of the row's bitmap
+  uint32_t rank0, n;     // rank of the item's first entry in the row, and its entries
+};
+
+// One block per row: popcounts of the groups, then one thread cuts them into
+// items. The other rows go to the rest list.
+__global__ void __launch_bounds__(256) k_item_plan(RowQueue q, const DevCounters* __restrict__ ctr,
+                                                   unsigned long long shares, const uint32_t* __restrict__ prod,
+                                                   const uint32_t* __restrict__ lo,
+                                                   const uint32_t* __restrict__ hi,
+                                                   const uint64_t* __restrict__ bm_off,
+                                                   const unsigned long long* __restrict__ cache,
+                                                   WinItem* __restrict__ items, uint32_t cap,
+                                                   uint32_t* __restrict__ rest, ItemCounters* __restrict__ ic) {
+  __shared__ uint16_t cnt[kBitmapWords / 32];
+  __shared__ uint16_t cut[kBitmapWords / 32 + 2];
+  __shared__ uint32_t s_base, s_n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t count = *q.count;
+  const unsigned long long heavy = ctr->num_prod[NB_BITMAP] / shares;
+  for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
+    const uint32_t row = q.rows[idx];
+    const uint64_t slot = bm_off[row];
+    const uint32_t nw = (uint32_t)(((uint64_t)hi[row] - lo[row] + 64) >> 6);
+    if (slot == ~0ull || (nw > kItemWideWords && prod[row] <= heavy)) {
+      if (threadIdx.x == 0) rest[atomicAdd(&ic->rest, 1u)] = row;
+      continue;
+    }
+    const uint32_t ng = (nw + 31) / 32;
+    for (uint32_t g = warp; g < ng; g += 8) {
+      const uint32_t w = g * 32 + lane;
+      const uint32_t c = __reduce_add_sync(kFull, w < nw ? (uint32_t)__popcll(cache[slot + w]) : 0u);
+      if (lane == 0) cnt[g] = (uint16_t)c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t items_n = 0, sum = 0, g0 = 0;
+      for (uint32_t g = 0; g < ng; ++g) {
+        const uint32_t c = cnt[g];
+        if (sum + c > (uint32_t)kItemV || g - g0 == (uint32_t)kItemGroups) {
+          cut[items_n++] = (uint16_t)g;
+          g0 = g;
+          sum = 0;
+        }
+        sum += c;
+      }
+      cut[items_n++] = (uint16_t)ng;
+      s_n = items_n;
+      s_base = atomicAdd(&ic->items, items_n);
+      if ((uint64_t)s_base + items_n > cap) {
+        // (the list is sized for every row; kept as a guard)
+        for (uint32_t i = s_base; i < cap; ++i) items[i] = WinItem{row, 0u, 0u, 0u, 0u};
+        rest[atomicAdd(&ic->rest, 1u)] = row;
+        s_n = 0;
+      }
+    }
+    __syncthreads();
+    // a warp per item: its rank is the popcount of the groups before it
+    for (uint32_t i = warp; i < s_n; i += 8) {
+      const uint32_t g0 = i ? cut[i - 1] : 0u, g1 = cut[i];
+      uint32_t before = 0, n = 0;
+      for (uint32_t g = lane; g < g1; g += 32) {
+        if (g < g0) before += cnt[g];
+        else n += cnt[g];
+      }
+      before = __reduce_add_sync(kFull, before);
+      n = __reduce_add_sync(kFull, n);
+      if (lane == 0) items[s_base + i] = WinItem{row, g0, g1, before, n};
+    }
+    __syncthreads();
+  }
+}
+
+// First position in [lo, hi) whose column is >= c (AFTER: > c), hi if there is
+// none, by quarters (three loads a step in flight) or, for BINARY, by halves:
+// with few searches in a block the steps' latency counts, with many the loads do.
+template <bool BINARY>
+__device__ __forceinline__ void item_search(const uint32_t* __restrict__ col, uint32_t ca, uint32_t cb, uint32_t& pl,
+                                            uint32_t ph, uint32_t& el, uint32_t eh) {
+  while (pl < ph || el < eh) {
+    const bool pa = pl < ph, ea = el < eh;
+    const uint32_t pn = ph - pl, en = eh - el;
+    if (BINARY) {
+      const uint32_t pm = pl + (pn >> 1), em = el + (en >> 1);
+      const uint32_t pc = pa ? col[pm] : 0u, ec = ea ? col[em] : 0u;
+      if (pa) {
+        if (pc < ca) pl = pm + 1; else ph = pm;
+      }
+      if (ea) {
+        if (ec <= cb) el = em + 1; else eh = em;
+      }
+    } else {
+      const uint32_t p1 = pl + (pn >> 2), p2 = pl + (pn >> 1), p3 = p2 + (pn >> 2);
+      const uint32_t e1 = el + (en >> 2), e2 = el + (en >> 1), e3 = e2 + (en >> 2);
+      uint32_t a1 = 0, a2 = 0, a3 = 0, b1 = 0, b2 = 0, b3 = 0;
+      if (pa) {
+        a1 = col[p1];
+        a2 = col[p2];
+        a3 = col[min(p3, ph - 1)];
+      }
+      if (ea) {
+        b1 = col[e1];
+        b2 = col[e2];
+        b3 = col[min(e3, eh - 1)];
+      }
+      if (pa) {
+        if (a2 < ca) {
+          pl = p2 + 1;
+          if (p3 < ph) {
+            if (a3 < ca) pl = max(pl, p3 + 1); else ph = max(pl, p3);
+          }
+        } else {
+          ph = p2;
+          if (a1 < ca) pl = min(p1 + 1, p2); else ph = p1;
+        }
+      }
+      if (ea) {
+        if (b2 <= cb) {
+          el = e2 + 1;
+          if (e3 < eh) {
+            if (b3 <= cb) el = max(el, e3 + 1); else eh = max(el, e3);
+          }
+        } else {
+          eh = e2;
+          if (b1 <= cb) el = min(e1 + 1, e2); else eh = e1;
+        }
+      }
+    }
+  }
+}
+
+struct ItemSmem {
+  double vals[kItemV];
+  uint32_t cols[kItemV];
+  unsigned long long words[kItemWords];
+  uint16_t wpre[kItemWords];
+  uint32_t gsum[kItemGroups];
+  EnumSmem<kBitmapThreads> e;
+  WinItem next;  // the next item and its row, fetched while the current one is worked on
+  uint64_t next_a0, next_a1, next_slot;
+  uint32_t next_lo, next_hi;
+  uint32_t idx[2];  // list positions, by turn
+};
+
+template <typename RP>
+__global__ void __launch_bounds__(kBitmapThreads, 1)
+    k_num_items(Csr<RP> A, Csr<RP> B, OutSpec o, DevCounters* __restrict__ ctr, const uint32_t* __restrict__ lo,
+                const uint32_t* __restrict__ hi, const uint64_t* __restrict__ bm_off,
+                const unsigned long long* __restrict__ cache, const WinItem* __restrict__ items, uint32_t item_cap,
+                ItemCounters* __restrict__ ic, uint32_t* __restrict__ c_col, double* __restrict__ c_val) {
+  constexpr int NT = kBitmapThreads;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ItemSmem& S = *reinterpret_cast<ItemSmem*>(smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < kItemV; i += NT) S.vals[i] = 0.0;
+  const uint32_t count = min(ic->items, item_cap);
+  // The chain item -> row -> row pointers and bitmap slot is fetched one item
+  // ahead, a few lanes loading one value each (2200 cycles an item when it
+  // was fetched at the item's start).
+  uint64_t value = 0;
+  auto load_item = [&](uint32_t idx) {
+    if (idx < count && tid < 5) value = reinterpret_cast<const uint32_t*>(items + idx)[tid];
+  };
+  auto store_item = [&]() {
+    if (tid < 5) reinterpret_cast<uint32_t*>(&S.next)[tid] = (uint32_t)value;
+  };
+  auto load_row = [&](uint32_t row) {
+    if (tid == 0) value = A.row_begin(row);
+    else if (tid == 1) value = A.row_end(row);
+    else if (tid == 2) value = bm_off[row];
+    else if (tid == 3) value = lo[row];
+    else if (tid == 4) value = hi[row];
+  };
+  auto store_row = [&]() {
+    if (tid < 3) (&S.next_a0)[tid] = value;
+    else if (tid < 5) (&S.next_lo)[tid - 3] = (uint32_t)value;
+  };
+  if (tid == 0) {
+    S.idx[1] = atomicAdd(&ic->cursor, 1u);
+    S.idx[0] = atomicAdd(&ic->cursor, 1u);
+  }
+  __syncthreads();
+  uint32_t idx = S.idx[1];
+  if (idx < count) {
+    load_item(idx);
+    store_item();
+    __syncthreads();
+    load_row(S.next.row);
+    store_row();
+  }
+  for (int turn = 0;; turn ^= 1) {
+    __syncthreads();
+    if (idx >= count) break;
+    const uint32_t next_idx = S.idx[turn];
+    uint32_t after_idx = 0;
+    if (tid == 0) after_idx = atomicAdd(&ic->cursor, 1u);
+    load_item(next_idx);
+    const WinItem it = S.next;
+    const uint32_t row = it.row;
+    const uint64_t rlo = S.next_lo, rhi = S.next_hi;
+    const uint64_t a0 = S.next_a0, a1 = S.next_a1, slot = S.next_slot;
+    const bool work = it.n != 0 && it.n <= (uint32_t)kItemV;  // (no entries, or a guard entry of the plan: none)
+    const uint32_t nw = (uint32_t)((rhi - rlo + 64) >> 6);
+    const uint32_t w0 = it.g0 * 32u, ng = work ? it.g1 - it.g0 : 0u;
+    // the window's words, 32 to a group, and the columns before each word
+    const unsigned long long* src = cache + slot;
+    uint32_t pre[kItemGroups / 32];
+#pragma unroll
+    for (int i = 0; i < kItemGroups / 32; ++i) {
+      const uint32_t g = (uint32_t)i * 32 + warp;
+      pre[i] = 0;
+      if (g < ng) {
+        const uint32_t w = w0 + g * 32 + lane;
+        const unsigned long long x = w < nw ? src[w] : 0ull;
+        S.words[g * 32 + lane] = x;
+        const uint32_t pc = (uint32_t)__popcll(x);
+        uint32_t y = pc;
+#pragma unroll
+        for (int sh = 1; sh < 32; sh <<= 1) {
+          const uint32_t z = __shfl_up_sync(kFull, y, sh);
+          if (lane >= sh) y += z;
+        }
+        pre[i] = y - pc;
+        if (lane == 31) S.gsum[g] = y;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      constexpr int PER = kItemGroups / 32;
+      uint32_t x[PER], sum = 0;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const uint32_t g = (uint32_t)lane * PER + i;
+        x[i] = g < ng ? S.gsum[g] : 0u;
+        sum += x[i];
+      }
+      uint32_t y = sum;
+#pragma unroll
+      for (int sh = 1; sh < 32; sh <<= 1) {
+        const uint32_t z = __shfl_up_sync(kFull, y, sh);
+        if (lane >= sh) y += z;
+      }
+      uint32_t run = y - sum;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const uint32_t g = (uint32_t)lane * PER + i;
+        if (g < ng) S.gsum[g] = run;
+        run += x[i];
+      }
+      store_item();
+      if (tid == 0) S.idx[turn ^ 1] = after_idx;
+    }
+    __syncthreads();
+    if (next_idx < count) load_row(S.next.row);
+#pragma unroll
+    for (int i = 0; i < kItemGroups / 32; ++i) {
+      const uint32_t g = (uint32_t)i * 32 + warp;
+      if (g < ng) S.wpre[g * 32 + lane] = (uint16_t)(S.gsum[g] + pre[i]);
+    }
+    // (ordered before the sums by the barriers of block_pack_chunk)
+    const uint64_t ca = rlo + 64ull * w0;
+    const bool first = it.g0 == 0, last = it.g1 * 32u >= nw;
+    const uint32_t ca32 = (uint32_t)ca, cb32 = (uint32_t)(last ? rhi : rlo + 64ull * 32 * it.g1 - 1);  // first, last column
+    const uint32_t span1 = cb32 - ca32;
+    auto accumulate = [&](uint32_t c, double v, bool ok) {
+      const uint32_t d = c - ca32;
+      if (ok && d <= span1) {
+        const uint32_t w = d >> 6;
+        const uint32_t r = S.wpre[w] + (uint32_t)__popcll(S.words[w] & ((1ull << (d & 63)) - 1ull));
+        if (r < (uint32_t)kItemV) {
+          S.cols[r] = c;
+          atomicAdd(&S.vals[r], v);
+        }
+      }
+    };
+    for (uint64_t c0 = work ? a0 : a1; c0 < a1; c0 += NT) {
+      const uint64_t k = c0 + tid;
+      unsigned long long b = 0;
+      uint32_t pl = 0, el = 0;
+      double av = 0.0;
+      if (k < a1) {
+        const uint32_t j = A.col[k];
+        av = A.val[k];
+        b = B.row_begin(j);
+        // the part of the B row inside the window (both ends searched together)
+        const uint32_t len = (uint32_t)(B.row_end(j) - b);
+        el = last ? len : 0u;
+        if (a1 - c0 <= 256)
+          item_search<false>(B.col + b, ca32, cb32, pl, first ? 0u : len, el, len);
+        else
+          item_search<true>(B.col + b, ca32, cb32, pl, first ? 0u : len, el, len);
+        el = max(el, pl);
+      }
+      block_pack_chunk<NT, true>(b + pl, el - pl, av, S.e);
+      block_run_chunk<NT, true>(B, S.e, accumulate);
+    }
+    if (next_idx < count) store_row();
+    idx = next_idx;
+    const uint64_t out = o.off[row] + it.rank0;
+    const uint32_t lim = o.cap[row];
+    const uint32_t n = !work || it.rank0 >= lim ? 0u : min(it.n, lim - it.rank0);
+    if (tid == 0 && work && last && it.rank0 + it.n != lim) raise_status(ctr, DEV_COUNT_MISMATCH, row);
+#pragma unroll 4
+    for (uint32_t i = tid; i < n; i += NT) {
+      c_col[out + i] = S.cols[i];
+      c_val[out + i] = S.vals[i];
+      S.vals[i] = 0.0;
+    }
+    for (uint32_t i = n + tid; work && i < it.n; i += NT) S.vals[i] = 0.0;
+  }
+}
+
 // ---------------------------------------------------------------- segment dispatch
 // Writes each row's dispatch slot: block i paints rows [iv[3i], iv[3i+1]) with
 // slot iv[3i+2]. Intervals are disjoint; unpainted rows keep slot 0.
@@ -2968,6 +3306,8 @@ __global__ void __launch_bounds__(256) k_row_bounds(uint64_t rows, const uint32_
 namespace {
 constexpr size_t kNumBitmapSmem = sizeof(BitmapNumSmem);
 constexpr size_t kWinNumSmem = sizeof(WinNumSmem);
+constexpr size_t kItemSmem = sizeof(ItemSmem);
+static_assert(kItemSmem <= 227 * 1024, "shared memory of one block");
 constexpr size_t kSymBitmapSmem = sizeof(BitmapSymSmem);
 template <int NT, int LOG2T>
 constexpr size_t num_hash_smem() { return sizeof(NumHashSmem<NT, LOG2T>); }
@@ -2997,6 +3337,7 @@ void set_attrs() {
   allow_smem(k_sym_bitmap<RP>, kSymBitmapSmem);
   allow_smem(k_num_bitmap<RP>, kNumBitmapSmem);
   allow_smem(k_num_window<RP>, kWinNumSmem);
+  allow_smem(k_num_items<RP>, kItemSmem);
   allow_smem(k_usp_fused<RP>, sizeof(UspSmem));
   allow_smem(k_sym_hash<RP, 128, 11>, sym_hash_smem<128, 11>());
   allow_smem(k_sym_hash<RP, 256, 13>, sym_hash_smem<256, 13>());
@@ -3044,6 +3385,9 @@ bool ensure_kernel_attributes(int dev) {
   }
   return true;
 }
+
+uint64_t item_capacity(uint64_t rows, uint64_t nnz) { return nnz / (kItemV - 2048) + 3 * rows + 1; }
+size_t item_bytes() { return sizeof(WinItem); }
 
 size_t window_scratch_words(int num_sms) { return (size_t)num_sms * (size_t)g_occ[K_NUM_WIN] * kBitmapWords; }
 
@@ -3251,6 +3595,19 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
       k_num_bitmap<RP><<<gsz, kBitmapThreads, kNumBitmapSmem, s>>>(A, B, wq, o, w.ctr, w.prod, w.lo, w.hi,
                                                                    w.bm_off, w.bm_cache, c_col, c_val, true);
     }
+  } else if (!o.count && w.items && w.bm_cache && (gsz = grid(K_NUM_BM, NB_BITMAP, 1))) {
+    // rows that the plan cuts into window items, and the others whole
+    cudaMemsetAsync(w.item_ctr, 0, sizeof(ItemCounters), s);
+    k_item_plan<<<std::min(8u * (unsigned)num_sms, counts ? counts[NB_BITMAP] : 8u * (unsigned)num_sms), 256, 0, s>>>(
+        queue(NB_BITMAP), w.ctr, 4ull * num_sms * (chunked ? w.chunks : 1), w.prod, w.lo, w.hi, w.bm_off, w.bm_cache,
+        static_cast<WinItem*>(w.items), w.item_cap, w.item_rest, w.item_ctr);
+    k_num_items<RP><<<num_sms, kBitmapThreads, kItemSmem, s>>>(A, B, o, w.ctr, w.lo, w.hi, w.bm_off, w.bm_cache,
+                                                               static_cast<const WinItem*>(w.items), w.item_cap,
+                                                               w.item_ctr, c_col, c_val);
+    const RowQueue rq{w.item_rest, &w.item_ctr->rest, &w.item_ctr->rest_cursor};
+    k_num_bitmap<RP><<<gsz, kBitmapThreads, kNumBitmapSmem, s>>>(A, B, rq, o, w.ctr, w.prod, w.lo, w.hi, w.bm_off,
+                                                                 w.bm_cache, c_col, c_val, false);
+    launched += 3;
   } else if ((gsz = grid(K_NUM_BM, NB_BITMAP, 1)) && ++launched) {
     k_num_bitmap<RP><<<gsz, kBitmapThreads, kNumBitmapSmem, s>>>(A, B, queue(NB_BITMAP), o, w.ctr, w.prod, w.lo,
                                                                  w.hi, w.bm_off, w.bm_cache, c_col, c_val, false);

@@ -205,6 +205,12 @@ struct ocean_handle {
   // fused ultra-sparse multiply: look-back state per tile (grow-only)
   unsigned long long* usp_tiles_buf = nullptr;
   uint64_t usp_tiles_cap = 0;
+  // window items of the numeric bitmap class (grow-only): item list, rest list, counters
+  unsigned char* item_buf = nullptr;
+  uint64_t item_buf_cap = 0;
+  uint32_t* item_rest = nullptr;
+  uint64_t item_rest_cap = 0;
+  ItemCounters* item_ctr = nullptr;
   // k_num_window: resume cursors per A entry and per-block bitmaps (grow-only)
   uint32_t* win_cursor = nullptr;
   uint64_t win_cursor_cap = 0;
@@ -234,6 +240,9 @@ struct ocean_handle {
     if (out_val) cudaFreeHost(out_val);
     if (cache_buf) cudaFree(cache_buf);
     if (usp_tiles_buf) cudaFree(usp_tiles_buf);
+    if (item_buf) cudaFree(item_buf);
+    if (item_rest) cudaFree(item_rest);
+    if (item_ctr) cudaFree(item_ctr);
     if (win_cursor) cudaFree(win_cursor);
     if (win_scratch) cudaFree(win_scratch);
     if (chunk_dev) cudaFree(chunk_dev);
@@ -635,6 +644,36 @@ void prepare_windows(ocean_handle* h, uint64_t a_nnz, unsigned bitmap_rows) {
   h->w.win_cursor = h->win_cursor;
   h->w.win_scratch = h->win_scratch;
   h->st.bm_kernel = 2;
+}
+
+// Buffers of the window items for the numeric bitmap class's saved rows. If
+// they cannot be allocated, the rows run whole in k_num_bitmap (no error).
+void prepare_items(ocean_handle* h, unsigned bitmap_rows, uint64_t bitmap_nnz) {
+  h->w.items = nullptr;
+  if (!h->w.bm_cache || bitmap_rows == 0 || h->cfg.numeric_windows) return;
+  const uint64_t cap = item_capacity(bitmap_rows, bitmap_nnz);
+  if (cap > 0xFFFFFFFFull) return;
+  auto try_grow = [](auto*& p, uint64_t& have, uint64_t need) {
+    if (p && have >= need) return true;
+    if (p) cudaFree(p);
+    p = nullptr;
+    have = 0;
+    if (cudaMalloc((void**)&p, need * sizeof(*p)) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return false;
+    }
+    have = need;
+    return true;
+  };
+  uint64_t one = h->item_ctr ? 1 : 0;
+  if (!try_grow(h->item_buf, h->item_buf_cap, cap * item_bytes()) ||
+      !try_grow(h->item_rest, h->item_rest_cap, bitmap_rows) || !try_grow(h->item_ctr, one, 1))
+    return;
+  h->w.items = h->item_buf;
+  h->w.item_cap = (uint32_t)cap;
+  h->w.item_rest = h->item_rest;
+  h->w.item_ctr = h->item_ctr;
 }
 
 // Phase 2 of the precise workflow: symbolic class kernels (exact counts into
@@ -1144,6 +1183,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         unsigned num_counts[NB_COUNT];
         for (int i = 0; i < NB_COUNT; ++i) num_counts[i] = h->h_ctr->num_count[i];
         prepare_windows(h, A.nnz, num_counts[NB_BITMAP]);
+        prepare_items(h, num_counts[NB_BITMAP], h->h_ctr->num_nnz[NB_BITMAP]);
         const OutSpec exact{h->w.rowptr64, h->w.row_nnz, nullptr, nullptr, nullptr};
         if (h->w.chunks) {
           st.launches += pipeline_numeric(h, A, B, exact, owner, nnz, bits, s);

@@ -106,6 +106,13 @@ enum DevError : unsigned int {
 
 constexpr uint32_t kUnknownCount = 0xFFFFFFFFu;
 
+// Queue of the window items of the numeric bitmap class, and of its rows that
+// are not cut into items.
+struct ItemCounters {
+  unsigned int items, cursor;
+  unsigned int rest, rest_cursor;
+};
+
 // A device-side list of rows rows[0 .. *count), taken one by one through *cursor.
 struct RowQueue {
   const uint32_t* rows;

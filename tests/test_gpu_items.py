@@ -1,0 +1,70 @@
+"""Window items of the numeric bitmap class (k_item_plan, k_num_items): rows
+with saved bitmaps cut by entries (more than 10240) and by words (more than
+2^19 columns), rows at the span where every row becomes items (2^18 columns),
+heavy rows among wide light ones, more A entries than one chunk (1024) and than
+the quarter search (256), 32- and 64-bit row pointers, row chunks of the
+host-buffer pipeline. Structure must match the oracle bit for bit, values
+within 1e-12 * sum |a*b| (at most 3000 FP64 terms per entry in another order:
+below 3000 * 2^-53 = 3.4e-13 of it)."""
+import numpy as np
+import pytest
+
+from research_b200 import matrices as M
+from research_b200.ocean import SpGEMM
+
+from test_gpu_parity import NUM_BINS, SYM_BINS, check, multiply_device
+from test_gpu_windows import heavy_mix
+
+pytestmark = pytest.mark.gpu
+
+FORCE = {"force_sym_bin": SYM_BINS["bitmap"], "force_num_bin": NUM_BINS["bitmap"]}
+
+
+@pytest.mark.parametrize("cols", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, 1 << 20])
+@pytest.mark.parametrize("wide_pointers", [False, True])
+def test_power_law_rows(cols, wide_pointers):
+    A, B = heavy_mix(b_rows=6000, cols=cols, seed=cols % 97)
+    if wide_pointers:
+        A, B = A.widened(), B.widened()
+    C, st = multiply_device(A, B)
+    check(A, B, C)
+    assert st["decision"]["bitmap_cache_used_bytes"] > 0
+    assert int(np.diff(C.rowptr.astype(np.int64)).max()) > 20480  # rows of several items
+
+
+@pytest.mark.parametrize("span", [64, 2048, 2049, 1 << 18, (1 << 19) + 1, 1 << 20])
+@pytest.mark.parametrize("entries", [1, 255, 256, 257, 1025])
+def test_item_edges(span, entries):
+    # one row of `entries` B rows of 9 columns, and single-entry rows beside it
+    rng = np.random.default_rng(span + entries)
+    r = np.repeat(np.arange(entries), 9)
+    c = rng.integers(0, span, r.size)
+    c[0], c[-1] = 0, span - 1
+    B = M.from_coo(entries, span, r, c, rng.uniform(-1, 1, r.size))
+    k = np.arange(entries)
+    A = M.from_coo(3, entries, np.r_[np.zeros(entries, int), 1, 2], np.r_[k, 0, entries - 1],
+                   rng.uniform(-1, 1, entries + 2))
+    C, _ = multiply_device(A, B, FORCE)
+    check(A, B, C)
+
+
+def test_items_hold_at_most_their_slots():
+    # one dense row: every column of 2^18, so the cuts fall at the slot limit
+    rng = np.random.default_rng(3)
+    span = 1 << 18
+    cols = rng.permutation(span)
+    B = M.from_coo(64, span, np.arange(span) % 64, cols, rng.uniform(-1, 1, span))
+    A = M.from_coo(2, 64, np.r_[np.zeros(64, int), np.ones(3, int)], np.r_[np.arange(64), 1, 5, 9],
+                   rng.uniform(-1, 1, 67))
+    C, _ = multiply_device(A, B)
+    check(A, B, C)
+    assert C.nnz > span
+
+
+@pytest.mark.parametrize("chunks", [2, 5])
+def test_items_in_the_host_pipeline(chunks):
+    A, B = heavy_mix(b_rows=6000, cols=1 << 18, seed=8)
+    g = SpGEMM({"host_pipeline_chunks": chunks, "host_pipeline_min_products": 1, "small_problem_nnz": 0})
+    C = g.multiply(A, B)
+    check(A, B, C)
+    assert g.get_stats()["decision"]["host_pipeline_chunks"] == chunks
