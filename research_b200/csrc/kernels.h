@@ -65,6 +65,9 @@ struct DevWork {
   uint32_t* chunk_bound = nullptr;
   unsigned* chunk_count = nullptr;
   unsigned* chunk_cursor = nullptr;
+  // the hash classes have narrow rows (host copies of the counters; 0: the
+  // narrow-row kernels are not launched and every row runs in its class kernel)
+  unsigned sym_narrow = 0, num_narrow = 0;
   // segment-driven dispatch: per-row policy slot (0: the call's policy,
   // 1 + SegClass: that segment class's policy); null: slot 0 for every row
   const uint8_t* row_pol = nullptr;

@@ -126,6 +126,15 @@ __device__ __forceinline__ uint32_t spread_index(uint32_t idx, uint32_t count, u
   return (uint32_t)(((uint64_t)idx * stride) % count);
 }
 
+// Rows of the hash classes that k_sym_narrow and k_num_narrow take: a span of
+// at most `most` columns, and B rows of 24 entries and more in the mean, which
+// keep the warp's lanes busy.
+constexpr uint32_t kNarrowSym = 4096;  // columns of a symbolic row
+constexpr uint32_t kNarrowNum = 1088;  // columns of a numeric row: 9.6 KB a warp, 20 warps per SM
+__device__ __forceinline__ bool narrow_row(uint64_t p, uint64_t anz, uint64_t span, uint32_t most) {
+  return span <= most && p >= 512 && p >= 24 * anz;
+}
+
 // ---------------------------------------------------------------- analysis
 // Row table of B for the analysis: first column, last column and length of
 // every row in one 16-byte entry, so an A entry costs one load of a table
@@ -236,7 +245,7 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
                                                   uint32_t* __restrict__ long_chunk_row, uint32_t chunk_cap,
                                                   const uint4* __restrict__ btab) {
   __shared__ unsigned long long s_anz[SB_COUNT], s_prod[SB_COUNT], s_words, s_tot;
-  __shared__ unsigned s_maxp, s_maxa, s_cnt[SB_COUNT];
+  __shared__ unsigned s_maxp, s_maxa, s_cnt[SB_COUNT], s_narrow;
   if (threadIdx.x < SB_COUNT) {
     s_anz[threadIdx.x] = 0ull;
     s_prod[threadIdx.x] = 0ull;
@@ -247,6 +256,7 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
     s_tot = 0ull;
     s_maxp = 0u;
     s_maxa = 0u;
+    s_narrow = 0u;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -296,6 +306,9 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
       }
     } else {
       b = analysis_write(row, a1 - a0, p, mn, mx, lb, prod, lo, hi, anz, maxb, row_nnz, bm_off, pols, row_pol);
+      if (b >= SB_HASH_S && b <= SB_HASH_L && pols.p[0].force_bin < 0 &&
+          narrow_row(p, a1 - a0, (uint64_t)mx - mn + 1, kNarrowSym))
+        s_narrow = 1u;
       // totals for stats and the workflow decision
       if (p) {
         atomicAdd(&s_tot, p);
@@ -349,6 +362,7 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
     if (s_tot) atomicAdd(&ctr->total_products, s_tot);
     if (s_maxp) atomicMax(&ctr->max_products, s_maxp);
     if (s_maxa) atomicMax(&ctr->max_a_nnz, s_maxa);
+    if (s_narrow) ctr->sym_narrow = 1u;
   }
 }
 
@@ -1230,6 +1244,183 @@ __device__ __forceinline__ void mark_bit(unsigned long long* bits, uint32_t c, b
   }
 }
 
+// ---------------------------------------------------------------- narrow rows
+// Rows of the hash classes with a narrow column span and long B rows (bands,
+// dense blocks), one warp per row: the warp takes the row's A entries one after
+// the other and walks each B row with its lanes, so the products of one step
+// have different columns and a plain load, add and store of the row's FP64
+// slots (one per column) takes the place of an atomic, and there is no block
+// barrier and no owner search. Four entries' loads are in flight. 2 * 10^5
+// banded rows (256/64, 7.2 * 10^8 products), one B200, block kernels -> these:
+// symbolic 1.9 -> 0.80 ms, numeric 4.4 -> 2.3 ms (315 G products/s; 20 warps
+// per SM by the slots, so the loads' latency is what is left); dense blocks
+// 256/64 of 57 entries a row, numeric 1.88 -> 1.3 ms.
+// op(column offset, value, same) for the products of A entries [a0, a1), by the
+// warp, step by step with a __syncwarp between; `same`: two lanes of the step
+// hold the same column (a B row that repeats one).
+template <bool VALS, typename RP, typename Op>
+__device__ __forceinline__ void warp_for_each_product(const Csr<RP>& A, const Csr<RP>& B, uint64_t a0, uint64_t a1,
+                                                      uint32_t rlo, uint32_t span1, Op&& op) {
+  const int lane = threadIdx.x & 31;
+  for (uint64_t k0 = a0; k0 < a1; k0 += 32) {
+    uint64_t bs = 0;
+    uint32_t len = 0;
+    double av = 0.0;
+    if (k0 + lane < a1) {
+      const uint32_t j = A.col[k0 + lane];
+      bs = B.row_begin(j);
+      len = (uint32_t)(B.row_end(j) - bs);
+      if (VALS) av = A.val[k0 + lane];
+    }
+    const int n = (int)min((uint64_t)32, a1 - k0);
+    for (int e0 = 0; e0 < n; e0 += 4) {
+      uint64_t b[4];
+      uint32_t l[4], most = 0;
+      double a[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        b[u] = __shfl_sync(kFull, bs, (e0 + u) & 31);
+        l[u] = __shfl_sync(kFull, len, (e0 + u) & 31);
+        a[u] = VALS ? __shfl_sync(kFull, av, (e0 + u) & 31) : 0.0;
+        if (e0 + u >= n) l[u] = 0;
+        most = max(most, l[u]);
+      }
+      for (uint32_t t0 = 0; t0 < most; t0 += 32) {
+        const uint32_t t = t0 + lane;
+        uint32_t c[4];
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          c[u] = kEmpty;
+          v[u] = 0.0;
+          if (t < l[u]) {
+            c[u] = B.col[b[u] + t];
+            if (VALS) v[u] = B.val[b[u] + t];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (t0 >= l[u]) continue;  // (warp-uniform)
+          bool same = false;
+          if (VALS) {
+            const uint32_t before = __shfl_up_sync(kFull, c[u], 1);
+            same = __any_sync(kFull, lane > 0 && c[u] != kEmpty && c[u] == before);
+          }
+          const uint32_t d = c[u] - rlo;
+          if (c[u] != kEmpty && d <= span1) op(d, a[u] * v[u], same);
+          __syncwarp();
+        }
+      }
+    }
+  }
+}
+
+constexpr int kNarrowWarps = 4;
+
+// What a class kernel knows of the narrow rows of its list: on, they are
+// skipped; when `done` counts the whole list, there is nothing else in it (a
+// list of 2 * 10^5 skipped rows costs a class kernel 0.3 ms). `done` is null
+// where a list is one of several row chunks.
+struct NarrowDone {
+  bool on;
+  const unsigned* done;
+  __device__ bool all(uint32_t count) const { return on && done && *done == count; }
+};
+
+template <typename RP>
+__global__ void __launch_bounds__(kNarrowWarps * 32)
+    k_sym_narrow(Csr<RP> A, Csr<RP> B, RowQueue q, const uint32_t* __restrict__ prod,
+                 const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi, uint32_t* __restrict__ row_nnz,
+                 unsigned* __restrict__ done) {
+  __shared__ __align__(16) uint8_t s_flag[kNarrowWarps][kNarrowSym];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* flag = s_flag[warp];
+  uint32_t* words = reinterpret_cast<uint32_t*>(flag);
+  for (uint32_t i = lane; i < kNarrowSym / 4; i += 32) words[i] = 0u;
+  __syncwarp();
+  unsigned mine = 0;
+  const uint32_t count = *q.count;
+  for (uint64_t idx = (uint64_t)blockIdx.x * kNarrowWarps + warp; idx < count; idx += (uint64_t)gridDim.x * kNarrowWarps) {
+    const uint32_t row = q.rows[idx];
+    const uint32_t rlo = lo[row], span1 = hi[row] - rlo;
+    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+    if (!narrow_row(prod[row], a1 - a0, (uint64_t)span1 + 1, kNarrowSym)) continue;
+    warp_for_each_product<false>(A, B, a0, a1, rlo, span1, [&](uint32_t d, double, bool) { flag[d] = 1; });
+    uint32_t n = 0;
+    for (uint32_t i = lane; i <= span1 >> 2; i += 32) {
+      n += __popc(words[i]);
+      words[i] = 0u;
+    }
+    n = __reduce_add_sync(kFull, n);
+    if (lane == 0) row_nnz[row] = n;
+    ++mine;
+    __syncwarp();
+  }
+  if (lane == 0 && mine) atomicAdd(done, mine);
+}
+
+template <typename RP>
+__global__ void __launch_bounds__(kNarrowWarps * 32)
+    k_num_narrow(Csr<RP> A, Csr<RP> B, RowQueue q, OutSpec o, DevCounters* __restrict__ ctr,
+                 const uint32_t* __restrict__ prod, const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
+                 uint32_t* __restrict__ c_col, double* __restrict__ c_val, unsigned* __restrict__ done) {
+  __shared__ double s_acc[kNarrowWarps][kNarrowNum];
+  __shared__ uint8_t s_flag[kNarrowWarps][kNarrowNum];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* acc = s_acc[warp];
+  uint8_t* flag = s_flag[warp];
+  const unsigned lt = lanemask_lt();
+  for (uint32_t i = lane; i < kNarrowNum; i += 32) {
+    acc[i] = 0.0;
+    flag[i] = 0;
+  }
+  __syncwarp();
+  unsigned mine = 0;
+  const uint32_t count = *q.count;
+  for (uint64_t idx = (uint64_t)blockIdx.x * kNarrowWarps + warp; idx < count; idx += (uint64_t)gridDim.x * kNarrowWarps) {
+    const uint32_t row = q.rows[idx];
+    const uint32_t rlo = lo[row], span1 = hi[row] - rlo;
+    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+    if (!narrow_row(prod[row], a1 - a0, (uint64_t)span1 + 1, kNarrowNum)) continue;
+    warp_for_each_product<true>(A, B, a0, a1, rlo, span1, [&](uint32_t d, double v, bool same) {
+      if (same) atomicAdd(&acc[d], v);
+      else acc[d] += v;
+      flag[d] = 1;
+    });
+    const uint32_t cap = o.cap[row];
+    const uint64_t off = o.off[row];
+    uint32_t lim = cap;
+    if (o.count) {  // estimated slots: the count decides whether the row is written
+      uint32_t n = 0;
+      for (uint32_t i = lane; i <= span1; i += 32) n += flag[i];
+      n = __reduce_add_sync(kFull, n);
+      int accept = 0;
+      if (lane == 0) accept = out_accept(o, ctr, row, n, cap);
+      if (!__shfl_sync(kFull, accept, 0)) lim = 0;
+    }
+    uint32_t at = 0;
+    for (uint32_t i0 = 0; i0 <= span1; i0 += 32) {
+      const uint32_t i = i0 + lane;  // (the slots are a multiple of 32)
+      const bool f = flag[i] != 0;
+      const unsigned m = __ballot_sync(kFull, f);
+      if (f) {
+        const uint32_t w = at + __popc(m & lt);
+        if (w < lim) {
+          c_col[off + w] = rlo + i;
+          c_val[off + w] = acc[i];
+        }
+        acc[i] = 0.0;
+        flag[i] = 0;
+      }
+      at += __popc(m);
+    }
+    if (!o.count && lane == 0) out_accept(o, ctr, row, at, cap);
+    ++mine;
+    __syncwarp();
+  }
+  if (lane == 0 && mine) atomicAdd(done, mine);
+}
+
 // ---------------------------------------------------------------- hash accumulators
 // Symbolic: one block per row. A row whose column span fits 32 columns per
 // table slot, with no more span words than products (so that clearing and
@@ -1250,12 +1441,13 @@ template <typename RP, int NT, int LOG2T>
 __global__ void __launch_bounds__(NT) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue q, DevCounters* __restrict__ ctr,
                                                  const uint32_t* __restrict__ prod, const uint32_t* __restrict__ maxb,
                                                  const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
-                                                 uint32_t* __restrict__ row_nnz) {
+                                                 uint32_t* __restrict__ row_nnz, NarrowDone narrow) {
   constexpr uint32_t T = 1u << LOG2T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SymHashSmem<NT, LOG2T>& S = *reinterpret_cast<SymHashSmem<NT, LOG2T>*>(smem_raw);
   const int tid = threadIdx.x;
   const uint32_t count = *q.count;
+  if (narrow.all(count)) return;
   const uint32_t* list = q.rows;
   for (;;) {
     if (tid == 0) S.s_idx = atomicAdd(q.cursor, 1u);
@@ -1267,6 +1459,10 @@ __global__ void __launch_bounds__(NT) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue 
     const uint32_t span1 = hi[row] - rlo;
     const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
     const uint32_t np = prod[row];
+    if (narrow.on && narrow_row(np, a1 - a0, (uint64_t)span1 + 1, kNarrowSym)) {  // k_sym_narrow's rows
+      __syncthreads();
+      continue;
+    }
     const int lg = group_lanes<NT>(a1 - a0, np, maxb[row]);
     unsigned cnt = 0;
     const uint32_t nw = (span1 >> 5) + 1;
@@ -1314,14 +1510,10 @@ __global__ void __launch_bounds__(NT) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue 
         }
         full |= probe == T;
       };
-      if (lg >= 0) {
-        __syncthreads();
-        group_for_each_product<NT, false>(A, B, a0, a1, lg, [&](uint32_t c, double) { insert(c); });
-      } else {
-        block_for_each_product<NT, false>(A, B, a0, a1, S.e, [&](uint32_t c, double, bool ok) {
-          if (ok) insert(c);
-        });
-      }
+      // (by groups, 2^18 uniform rows of 32: 1.94 ms against 1.70 ms)
+      block_for_each_product<NT, false>(A, B, a0, a1, S.e, [&](uint32_t c, double, bool ok) {
+        if (ok) insert(c);
+      });
       if (full) raise_status(ctr, DEV_TABLE_FULL, row);
     }
     const unsigned long long total = block_sum_u64<NT>(cnt, S.red);
@@ -1389,7 +1581,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B
                                                  DevCounters* __restrict__ ctr, const uint32_t* __restrict__ prod,
                                                  const uint32_t* __restrict__ maxb, const uint32_t* __restrict__ lo,
                                                  const uint32_t* __restrict__ hi, uint32_t* __restrict__ c_col,
-                                                 double* __restrict__ c_val) {
+                                                 double* __restrict__ c_val, NarrowDone narrow) {
   constexpr int NW = NT / 32;
   constexpr int P = kUnroll * NT;
   static_assert(kUnroll == 4, "one 16-byte group of bucket counts per thread");
@@ -1399,6 +1591,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const unsigned lt = lanemask_lt();
   const uint32_t count = *q.count;
+  if (narrow.all(count)) return;
   const uint32_t* list = q.rows;
   for (;;) {
     if (tid == 0) S.s_idx = atomicAdd(q.cursor, 1u);
@@ -1412,7 +1605,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B
     const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
     const uint32_t cap = o.cap[row];
     const uint64_t off = o.off[row];
-    if (span1 >= (uint32_t)kBitmapBits) {  // k_num_hash's rows
+    if (span1 >= (uint32_t)kBitmapBits ||  // k_num_hash's rows
+        (narrow.on && narrow_row(np, a1 - a0, (uint64_t)span1 + 1, kNarrowNum))) {  // k_num_narrow's rows
       __syncthreads();
       continue;
     }
@@ -2944,6 +3138,9 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       if (b == NB_BITMAP && (uint64_t)hi[i] - lo[i] + 1 > kBitmapBits) atomicAdd(&ctr->num_wide, 1u);
       aq[q] = anz[i];
       pq[q] = p;
+      if ((b == NB_HASH_S || b == NB_HASH_M) && pols.p[0].force_bin < 0 &&
+          narrow_row(p, aq[q], (uint64_t)hi[i] - lo[i] + 1, kNarrowNum))
+        ctr->num_narrow = 1u;
     }
     bq[q] = b;
     rq[q] = (uint32_t)i;
@@ -3465,18 +3662,30 @@ int launch_symbolic(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, int nu
   mark(SB_ESC4);
   if ((gsz = grid(K_SYM_ESC4, SB_ESC4, 8)) && ++launched)
     k_sym_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(SB_ESC4), w.ctr, w.row_nnz);
+  // narrow rows of the hash classes, a warp each (timed with the small-hash class)
+  auto narrow = [&](int cls) {
+    if (w.sym_narrow && (!counts || counts[cls]) && ++launched)
+      k_sym_narrow<RP><<<9 * num_sms, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), w.prod, w.lo, w.hi, w.row_nnz,
+                                                                  w.ctr->sym_narrow_done + cls);
+  };
   mark(SB_HASH_S);
+  narrow(SB_HASH_S);
+  narrow(SB_HASH_M);
+  narrow(SB_HASH_L);
   if ((gsz = grid(K_SYM_S, SB_HASH_S, 1)) && ++launched)
     k_sym_hash<RP, 128, 11><<<gsz, 128, sym_hash_smem<128, 11>(), s>>>(A, B, queue(SB_HASH_S), w.ctr, w.prod, w.maxb,
-                                                                       w.lo, w.hi, w.row_nnz);
+                                                                       w.lo, w.hi, w.row_nnz,
+                                                                       NarrowDone{w.sym_narrow != 0, w.ctr->sym_narrow_done + SB_HASH_S});
   mark(SB_HASH_M);
   if ((gsz = grid(K_SYM_M, SB_HASH_M, 1)) && ++launched)
     k_sym_hash<RP, 256, 13><<<gsz, 256, sym_hash_smem<256, 13>(), s>>>(A, B, queue(SB_HASH_M), w.ctr, w.prod, w.maxb,
-                                                                       w.lo, w.hi, w.row_nnz);
+                                                                       w.lo, w.hi, w.row_nnz,
+                                                                       NarrowDone{w.sym_narrow != 0, w.ctr->sym_narrow_done + SB_HASH_M});
   mark(SB_HASH_L);
   if ((gsz = grid(K_SYM_L, SB_HASH_L, 1)) && ++launched)
     k_sym_hash<RP, 512, 15><<<gsz, 512, sym_hash_smem<512, 15>(), s>>>(A, B, queue(SB_HASH_L), w.ctr, w.prod, w.maxb,
-                                                                       w.lo, w.hi, w.row_nnz);
+                                                                       w.lo, w.hi, w.row_nnz,
+                                                                       NarrowDone{w.sym_narrow != 0, w.ctr->sym_narrow_done + SB_HASH_L});
   mark(SB_BITMAP);
   if ((gsz = grid(K_SYM_BM, SB_BITMAP, 1)) && ++launched)
     k_sym_bitmap<RP><<<gsz, kBitmapThreads, kSymBitmapSmem, s>>>(A, B, queue(SB_BITMAP), w.ctr, w.prod, w.lo, w.hi,
@@ -3559,24 +3768,37 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
   mark(NB_ESC4);
   if ((gsz = grid(K_NUM_ESC4, NB_ESC4, 8)) && ++launched)
     k_num_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(NB_ESC4), o, w.ctr, c_col, c_val);
+  auto narrow_done = [&](int cls) {
+    return NarrowDone{w.num_narrow != 0, chunked ? nullptr : w.ctr->num_narrow_done + cls};
+  };
+  auto narrow = [&](int cls) {
+    if (w.num_narrow && (!counts || counts[cls]) && ++launched)
+      k_num_narrow<RP><<<5 * num_sms, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), o, w.ctr, w.prod, w.lo, w.hi, c_col,
+                                                                 c_val, w.ctr->num_narrow_done + cls);
+  };
   mark(NB_HASH_S);
+  narrow(NB_HASH_S);
   if ((gsz = grid(K_NUM_S, NB_HASH_S, 1)) && ++launched)
     k_num_rank<RP, 128, 512><<<gsz, 128, num_rank_smem<128, 512>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.prod, w.maxb,
-                                                                  w.lo, w.hi, c_col, c_val);
+                                                                  w.lo, w.hi, c_col, c_val,
+                                                                  narrow_done(NB_HASH_S));
   if (wide && gsz && ++launched)
     k_num_hash<RP, 128, 10><<<gsz, 128, num_hash_smem<128, 10>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.lo, w.hi,
                                                                   c_col, c_val);
   mark(NB_HASH_M);
+  narrow(NB_HASH_M);
   if ((gsz = grid(K_NUM_M, NB_HASH_M, 1)) && ++launched)
     k_num_rank<RP, 256, 2048><<<gsz, 256, num_rank_smem<256, 2048>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.prod, w.maxb,
-                                                                  w.lo, w.hi, c_col, c_val);
+                                                                  w.lo, w.hi, c_col, c_val,
+                                                                  narrow_done(NB_HASH_M));
   if (wide && gsz && ++launched)
     k_num_hash<RP, 256, 12><<<gsz, 256, num_hash_smem<256, 12>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.lo, w.hi,
                                                                   c_col, c_val);
   mark(NB_HASH_L);
   if ((gsz = grid(K_NUM_L, NB_HASH_L, 1)) && ++launched)
     k_num_rank<RP, 512, 4096><<<gsz, 512, num_rank_smem<512, 4096>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.prod, w.maxb,
-                                                                  w.lo, w.hi, c_col, c_val);
+                                                                  w.lo, w.hi, c_col, c_val,
+                                                                  NarrowDone{false, nullptr});
   if (wide && gsz && ++launched)
     k_num_hash<RP, 512, 13><<<gsz, 512, num_hash_smem<512, 13>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.lo, w.hi,
                                                                   c_col, c_val);

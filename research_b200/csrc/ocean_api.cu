@@ -722,6 +722,7 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
       }
     }
   }
+  h->w.sym_narrow = h->h_ctr->sym_narrow;
   // per-class boundary events only when stage timing is asked for (each record costs device time)
   const bool track = h->cfg.track_stage_times;
   h->st.launches += launch_symbolic(A, B, h->w, h->num_sms, s, track ? h->ev + EV_SYM0 : nullptr,
@@ -1143,6 +1144,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         for (int i = 0; i < NB_COUNT; ++i) num_counts[i] = h->h_ctr->num_count[i];
         const OutSpec est_out{h->w.est_off, h->w.est, h->w.cnt, h->w.ovf, &h->w.ctr->overflow_n};
         st.bm_kernel = num_counts[NB_BITMAP] ? 1 : 0;
+        h->w.num_narrow = class_counts ? h->h_ctr->num_narrow : 0u;
         st.launches += launch_numeric(A, B, h->w, est_out, (uint32_t*)t_col, (double*)t_val, h->num_sms, s,
                                       track ? h->ev + EV_NUM0 : nullptr, class_counts ? num_counts : nullptr);
         if (track) h->ev_mask |= ((1ull << (NB_COUNT + 1)) - 1) << EV_NUM0;
@@ -1184,6 +1186,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         for (int i = 0; i < NB_COUNT; ++i) num_counts[i] = h->h_ctr->num_count[i];
         prepare_windows(h, A.nnz, num_counts[NB_BITMAP]);
         prepare_items(h, num_counts[NB_BITMAP], h->h_ctr->num_nnz[NB_BITMAP]);
+        h->w.num_narrow = h->h_ctr->num_narrow;
         const OutSpec exact{h->w.rowptr64, h->w.row_nnz, nullptr, nullptr, nullptr};
         if (h->w.chunks) {
           st.launches += pipeline_numeric(h, A, B, exact, owner, nnz, bits, s);

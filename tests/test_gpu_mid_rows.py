@@ -123,3 +123,53 @@ def test_uneven_b_rows_take_the_balanced_enumeration():
     for num in ("hash_m", "hash_l"):
         for sym in CLASSES:
             _run(A, B, num, sym if sym != "hash_s" else "hash_m")
+
+
+def _narrow(rows, width, per_row, seed, repeat=False):
+    """Square-ish product whose rows span exactly `width` columns: every A row
+    references `per_row` B rows of 40 columns inside the width."""
+    rng = np.random.default_rng(seed)
+    nb = 64
+    r, c = [], []
+    for i in range(nb):
+        k = np.sort(rng.choice(width, min(40, width), replace=False))
+        if i == 0:
+            k[0], k[-1] = 0, width - 1
+        if repeat and i % 3 == 0:
+            k[1::2] = k[0:len(k) - 1:2][:len(k[1::2])]  # every column twice
+            k[0], k[-1] = 0, width - 1
+            k = np.sort(k)
+        r += [i] * len(k)
+        c += list(k)
+    B = M.from_coo(nb, width + 9, r, c, rng.uniform(-1, 1, len(r)), sum_duplicates=False)
+    ar = np.repeat(np.arange(rows), per_row)
+    ac = np.concatenate([np.r_[0, 1 + rng.choice(nb - 1, per_row - 1, replace=False)] for _ in range(rows)])
+    return M.from_coo(rows, nb, ar, ac, rng.uniform(-1, 1, ar.size)), B
+
+
+@pytest.mark.parametrize("width", [41, 1024, 1087, 1088, 1089, 4095, 4096, 4097])
+@pytest.mark.parametrize("per_row", [13, 31, 32, 33, 60])
+def test_narrow_rows_run_a_warp_each(width, per_row):
+    # spans at the limits of the numeric (1088) and symbolic (4096) narrow kernels,
+    # A rows around one warp's entries; 13 * 40 products is just past the 512 they need
+    A, B = _narrow(50, width, per_row, width + per_row)
+    for a, b in ((A, B), (A.widened(), B.widened())):
+        C, _ = multiply_device(a, b)
+        check(a, b, C)
+
+
+@pytest.mark.parametrize("wf", [0, 1])
+def test_narrow_rows_with_repeated_columns(wf):
+    # B rows that hold a column twice: two lanes of one step meet
+    A, B = _narrow(40, 700, 40, 9, repeat=True)
+    C, st = multiply_device(A, B, {"force_workflow": wf})
+    check(A, B, C)
+    assert st["decision"]["workflow"] == wf
+
+
+@pytest.mark.parametrize("scale", [0.3, 1.0])
+def test_narrow_rows_in_the_estimation_workflow(scale):
+    A = M.block_diagonal(20000, 256, 64, seed=2)
+    C, st = multiply_device(A, A, {"force_workflow": 1, "estimate_scale": scale})
+    check(A, A, C)
+    assert st["decision"]["workflow"] == 1
