@@ -127,12 +127,16 @@ __device__ __forceinline__ uint32_t spread_index(uint32_t idx, uint32_t count, u
 }
 
 // Rows of the hash classes that k_sym_narrow and k_num_narrow take: a span of
-// at most `most` columns, and B rows of 24 entries and more in the mean, which
-// keep the warp's lanes busy.
+// at most `most` columns, more products than the register classes hold, and B
+// rows of 8 entries and more in the mean. A warp step then has a quarter of its
+// lanes busy, which still beats a block's barriers (131072 rows, whole
+// multiply, in their block class -> a warp each: bands of 12 entries a row
+// 664 -> 530 us, 16 entries 968 -> 569 us, 24 entries 1334 -> 713 us; blocks of
+// 16 entries 946 -> 553 us, 32 entries 951 -> 942 us).
 constexpr uint32_t kNarrowSym = 4096;  // columns of a symbolic row
 constexpr uint32_t kNarrowNum = 1088;  // columns of a numeric row: 9.6 KB a warp, 20 warps per SM
 __device__ __forceinline__ bool narrow_row(uint64_t p, uint64_t anz, uint64_t span, uint32_t most) {
-  return span <= most && p >= 512 && p >= 24 * anz;
+  return span <= most && p > 128 && p >= 8 * anz;
 }
 
 // ---------------------------------------------------------------- analysis

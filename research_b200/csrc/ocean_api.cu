@@ -1590,6 +1590,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
     batch_readback(b, s);
     const DevCounters& k = *b->h_ctr;
     for (int i = 0; i < SB_COUNT; ++i) b->sym_counts[i] = k.sym_count[i];
+    w.sym_narrow = k.sym_narrow;
     b->products = k.total_products;
     const Config& c = b->cfg;
     const double avg = A.rows ? (double)k.total_products / (double)A.rows : 0.0;
@@ -1615,6 +1616,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
       batch_readback(b, s);
       b->c_nnz = b->h_ctr->total_nnz;
       for (int i = 0; i < NB_COUNT; ++i) b->num_counts[i] = b->h_ctr->num_count[i];
+      w.num_narrow = b->h_ctr->num_narrow;
     } else {
       launch_batch_guard(w.ctr, &w.ctr->total_nnz, b->c_nnz, s);
       launched += 1;
@@ -1640,6 +1642,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
       batch_readback(b, s);
       b->total_est = b->h_ctr->total_est;
       for (int i = 0; i < NB_COUNT; ++i) b->num_counts[i] = b->h_ctr->num_count[i];
+      w.num_narrow = b->h_ctr->num_narrow;
       OCEAN_CUDA(cudaMalloc((void**)&b->t_col, std::max<uint64_t>(b->total_est, 1) * 4));
       OCEAN_CUDA(cudaMalloc((void**)&b->t_val, std::max<uint64_t>(b->total_est, 1) * 8));
     } else {

@@ -125,14 +125,14 @@ def test_uneven_b_rows_take_the_balanced_enumeration():
             _run(A, B, num, sym if sym != "hash_s" else "hash_m")
 
 
-def _narrow(rows, width, per_row, seed, repeat=False):
-    """Square-ish product whose rows span exactly `width` columns: every A row
-    references `per_row` B rows of 40 columns inside the width."""
+def _narrow(rows, width, per_row, seed, repeat=False, length=40):
+    """Product whose rows span exactly `width` columns: every A row references
+    `per_row` B rows of `length` columns inside the width."""
     rng = np.random.default_rng(seed)
     nb = 64
     r, c = [], []
     for i in range(nb):
-        k = np.sort(rng.choice(width, min(40, width), replace=False))
+        k = np.sort(rng.choice(width, min(length, width), replace=False))
         if i == 0:
             k[0], k[-1] = 0, width - 1
         if repeat and i % 3 == 0:
@@ -148,11 +148,12 @@ def _narrow(rows, width, per_row, seed, repeat=False):
 
 
 @pytest.mark.parametrize("width", [41, 1024, 1087, 1088, 1089, 4095, 4096, 4097])
-@pytest.mark.parametrize("per_row", [13, 31, 32, 33, 60])
-def test_narrow_rows_run_a_warp_each(width, per_row):
+@pytest.mark.parametrize("per_row,length", [(4, 33), (16, 8), (17, 8), (31, 40), (32, 40), (33, 40), (60, 7), (60, 9)])
+def test_narrow_rows_run_a_warp_each(width, per_row, length):
     # spans at the limits of the numeric (1088) and symbolic (4096) narrow kernels,
-    # A rows around one warp's entries; 13 * 40 products is just past the 512 they need
-    A, B = _narrow(50, width, per_row, width + per_row)
+    # A rows around one warp's entries, products around the 128 of the register
+    # classes, B rows around the 8 entries that the narrow kernels ask for
+    A, B = _narrow(50, width, per_row, width + per_row, length=length)
     for a, b in ((A, B), (A.widened(), B.widened())):
         C, _ = multiply_device(a, b)
         check(a, b, C)
@@ -173,3 +174,16 @@ def test_narrow_rows_in_the_estimation_workflow(scale):
     C, st = multiply_device(A, A, {"force_workflow": 1, "estimate_scale": scale})
     check(A, A, C)
     assert st["decision"]["workflow"] == 1
+
+
+def test_narrow_rows_in_a_batch():
+    # a captured plan runs its narrow rows a warp each, run after run
+    from research_b200.ocean import Batch, DeviceCSR, SpGEMM
+    ms = [M.banded(3000, 30, 16, seed=1), M.block_diagonal(2000, 100, 20, seed=2), M.uniform_random(1500, 14, seed=3)]
+    for cfg in ({"force_workflow": 0}, {"use_learned_estimator": True}):
+        g = SpGEMM(cfg)
+        plan = Batch(g, [DeviceCSR.from_host(m) for m in ms])
+        for _ in range(3):
+            for m, c in zip(ms, plan.run()):
+                check(m, m, c.download())
+        plan.close()
