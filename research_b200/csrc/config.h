@@ -188,7 +188,7 @@ struct Config {
   int force_num_bin = -1;         // testing: put every non-empty row in one numeric class
   bool sync_on_return = true;     // check device status before returning
   double bitmap_cache_fraction = 0.25;  // share of free device memory the saved row bitmaps may use
-  int small_problem_nnz = 1 << 20;      // A with at most this many entries: no read-back after analysis
+  int small_problem_nnz = 1 << 20;      // A with at most this many entries: precise workflow unless forced
   int spin_wait_us = 2000;              // poll the stream this long before a blocking synchronize
   int force_workflow = -1;              // -1 auto; 0 precise, 1 estimation (HLL), 2 ultra-sparse, 3 fat
   double estimate_scale = 1.0;          // multiplies the HLL expansion (testing: < 1 forces overflows)

@@ -65,8 +65,9 @@ struct DevWork {
   uint32_t* chunk_bound = nullptr;
   unsigned* chunk_count = nullptr;
   unsigned* chunk_cursor = nullptr;
-  // the hash classes have narrow rows (host copies of the counters; 0: the
-  // narrow-row kernels are not launched and every row runs in its class kernel)
+  // symbolic hash classes (bits) that may have narrow rows, and whether the
+  // numeric ones have any (0: the narrow-row kernels are not launched and every
+  // row runs in its class kernel)
   unsigned sym_narrow = 0, num_narrow = 0;
   // segment-driven dispatch: per-row policy slot (0: the call's policy,
   // 1 + SegClass: that segment class's policy); null: slot 0 for every row
@@ -213,6 +214,13 @@ int launch_row_bounds(const DevWork& w, uint32_t* out, cudaStream_t s);
 // every entry point that may be first on a device; false: bad ordinal).
 void configure_kernel_attributes();
 bool ensure_kernel_attributes(int dev);
+
+// Symbolic hash classes (bits) whose list k_sym_narrow looks through before the
+// class kernel: at least 1024 rows, whose B rows have 8 entries and more in the
+// mean. Decided from the class sums: a test of every row in the analysis cost
+// the row sizing of the 2^21 power-law graph 9 us of 2265, a look through the
+// list of 2^18 rows without a narrow one costs 10 us of 7500.
+unsigned sym_narrow_classes(const DevCounters& c);
 
 // Most window items of `rows` bitmap-class rows with `nnz` output entries, and
 // the bytes of one.

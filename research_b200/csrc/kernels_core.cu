@@ -11,9 +11,9 @@
 //
 // Design: every row class runs as a persistent kernel whose blocks pull rows
 // from a device-side class list, so the kernels need no bin count from the
-// host. The host reads back the class sizes after the analysis (large inputs
-// only, to size the grids and the bitmap cache) and the total output count
-// (to allocate C).
+// host. The host reads back the class sizes after the analysis (to launch only
+// the classes that have rows, size the grids and the bitmap cache) and the total
+// output count (to allocate C).
 // Numeric kernels write each row already sorted straight into its final place
 // in C, so there is no temporary output buffer and no separate sort/copy pass.
 #include <algorithm>
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
                                                   uint32_t* __restrict__ long_chunk_row, uint32_t chunk_cap,
                                                   const uint4* __restrict__ btab) {
   __shared__ unsigned long long s_anz[SB_COUNT], s_prod[SB_COUNT], s_words, s_tot;
-  __shared__ unsigned s_maxp, s_maxa, s_cnt[SB_COUNT], s_narrow;
+  __shared__ unsigned s_maxp, s_maxa, s_cnt[SB_COUNT];
   if (threadIdx.x < SB_COUNT) {
     s_anz[threadIdx.x] = 0ull;
     s_prod[threadIdx.x] = 0ull;
@@ -260,7 +260,6 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
     s_tot = 0ull;
     s_maxp = 0u;
     s_maxa = 0u;
-    s_narrow = 0u;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -310,9 +309,6 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
       }
     } else {
       b = analysis_write(row, a1 - a0, p, mn, mx, lb, prod, lo, hi, anz, maxb, row_nnz, bm_off, pols, row_pol);
-      if (b >= SB_HASH_S && b <= SB_HASH_L && pols.p[0].force_bin < 0 &&
-          narrow_row(p, a1 - a0, (uint64_t)mx - mn + 1, kNarrowSym))
-        s_narrow = 1u;
       // totals for stats and the workflow decision
       if (p) {
         atomicAdd(&s_tot, p);
@@ -366,7 +362,6 @@ __global__ void __launch_bounds__(256, sizeof(RP) == 4 ? 8 : 6) k_analysis(Csr<R
     if (s_tot) atomicAdd(&ctr->total_products, s_tot);
     if (s_maxp) atomicMax(&ctr->max_products, s_maxp);
     if (s_maxa) atomicMax(&ctr->max_a_nnz, s_maxa);
-    if (s_narrow) ctr->sym_narrow = 1u;
   }
 }
 
@@ -3609,6 +3604,13 @@ bool ensure_kernel_attributes(int dev) {
 uint64_t item_capacity(uint64_t rows, uint64_t nnz) { return nnz / (kItemV - 2048) + 3 * rows + 1; }
 size_t item_bytes() { return sizeof(WinItem); }
 
+unsigned sym_narrow_classes(const DevCounters& c) {
+  unsigned mask = 0;
+  for (int k = SB_HASH_S; k <= SB_HASH_L; ++k)
+    if (c.sym_count[k] >= 1024 && c.sym_prod[k] >= 8 * c.sym_anz[k]) mask |= 1u << k;
+  return mask;
+}
+
 size_t window_scratch_words(int num_sms) { return (size_t)num_sms * (size_t)g_occ[K_NUM_WIN] * kBitmapWords; }
 
 template <typename RP>
@@ -3686,8 +3688,11 @@ int launch_symbolic(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, int nu
   if ((gsz = grid(K_SYM_ESC4, SB_ESC4, 8)) && ++launched)
     k_sym_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(SB_ESC4), w.ctr, w.row_nnz);
   // narrow rows of the hash classes, a warp each (timed with the small-hash class)
+  auto narrow_done = [&](int cls) {
+    return NarrowDone{((w.sym_narrow >> cls) & 1u) != 0, w.ctr->sym_narrow_done + cls};
+  };
   auto narrow = [&](int cls) {
-    if (w.sym_narrow && (!counts || counts[cls]) && ++launched)
+    if (((w.sym_narrow >> cls) & 1u) && ++launched)
       k_sym_narrow<RP><<<9 * num_sms, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), w.prod, w.lo, w.hi, w.row_nnz,
                                                                   w.ctr->sym_narrow_done + cls);
   };
@@ -3698,17 +3703,17 @@ int launch_symbolic(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, int nu
   if ((gsz = grid(K_SYM_S, SB_HASH_S, 1)) && ++launched)
     k_sym_hash<RP, 128, 11><<<gsz, 128, sym_hash_smem<128, 11>(), s>>>(A, B, queue(SB_HASH_S), w.ctr, w.prod, w.maxb,
                                                                        w.lo, w.hi, w.row_nnz,
-                                                                       NarrowDone{w.sym_narrow != 0, w.ctr->sym_narrow_done + SB_HASH_S});
+                                                                       narrow_done(SB_HASH_S));
   mark(SB_HASH_M);
   if ((gsz = grid(K_SYM_M, SB_HASH_M, 1)) && ++launched)
     k_sym_hash<RP, 256, 13><<<gsz, 256, sym_hash_smem<256, 13>(), s>>>(A, B, queue(SB_HASH_M), w.ctr, w.prod, w.maxb,
                                                                        w.lo, w.hi, w.row_nnz,
-                                                                       NarrowDone{w.sym_narrow != 0, w.ctr->sym_narrow_done + SB_HASH_M});
+                                                                       narrow_done(SB_HASH_M));
   mark(SB_HASH_L);
   if ((gsz = grid(K_SYM_L, SB_HASH_L, 1)) && ++launched)
     k_sym_hash<RP, 512, 15><<<gsz, 512, sym_hash_smem<512, 15>(), s>>>(A, B, queue(SB_HASH_L), w.ctr, w.prod, w.maxb,
                                                                        w.lo, w.hi, w.row_nnz,
-                                                                       NarrowDone{w.sym_narrow != 0, w.ctr->sym_narrow_done + SB_HASH_L});
+                                                                       narrow_done(SB_HASH_L));
   mark(SB_BITMAP);
   if ((gsz = grid(K_SYM_BM, SB_BITMAP, 1)) && ++launched)
     k_sym_bitmap<RP><<<gsz, kBitmapThreads, kSymBitmapSmem, s>>>(A, B, queue(SB_BITMAP), w.ctr, w.prod, w.lo, w.hi,

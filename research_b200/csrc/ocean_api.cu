@@ -722,7 +722,7 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
       }
     }
   }
-  h->w.sym_narrow = h->h_ctr->sym_narrow;
+  h->w.sym_narrow = h->cfg.force_sym_bin < 0 ? sym_narrow_classes(*h->h_ctr) : 0u;
   // per-class boundary events only when stage timing is asked for (each record costs device time)
   const bool track = h->cfg.track_stage_times;
   h->st.launches += launch_symbolic(A, B, h->w, h->num_sms, s, track ? h->ev + EV_SYM0 : nullptr,
@@ -1590,7 +1590,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
     batch_readback(b, s);
     const DevCounters& k = *b->h_ctr;
     for (int i = 0; i < SB_COUNT; ++i) b->sym_counts[i] = k.sym_count[i];
-    w.sym_narrow = k.sym_narrow;
+    w.sym_narrow = b->cfg.force_sym_bin < 0 ? sym_narrow_classes(k) : 0u;
     b->products = k.total_products;
     const Config& c = b->cfg;
     const double avg = A.rows ? (double)k.total_products / (double)A.rows : 0.0;

@@ -72,7 +72,7 @@ struct DevCounters {
   unsigned int usp_tile;     // fused ultra-sparse multiply: tiles handed out
   unsigned int num_long;     // rows of A listed as long (more than kLongRowEntries entries)
   unsigned int long_chunks;  // chunks of kLongChunk A entries of the listed rows
-  unsigned int sym_narrow;   // the symbolic hash classes have rows for k_sym_narrow
+  unsigned int pad[1];
   unsigned int num_narrow;   // the numeric hash classes have rows for k_num_narrow
   unsigned int sym_narrow_done[SB_COUNT];  // rows of each class that k_sym_narrow has counted
   unsigned int num_narrow_done[NB_COUNT];  // rows of each class that k_num_narrow has written

@@ -153,7 +153,8 @@ def test_narrow_rows_run_a_warp_each(width, per_row, length):
     # spans at the limits of the numeric (1088) and symbolic (4096) narrow kernels,
     # A rows around one warp's entries, products around the 128 of the register
     # classes, B rows around the 8 entries that the narrow kernels ask for
-    A, B = _narrow(50, width, per_row, width + per_row, length=length)
+    # (1024 rows in the list: the fewest that the symbolic one looks through)
+    A, B = _narrow(1024, width, per_row, width + per_row, length=length)
     for a, b in ((A, B), (A.widened(), B.widened())):
         C, _ = multiply_device(a, b)
         check(a, b, C)
@@ -162,7 +163,7 @@ def test_narrow_rows_run_a_warp_each(width, per_row, length):
 @pytest.mark.parametrize("wf", [0, 1])
 def test_narrow_rows_with_repeated_columns(wf):
     # B rows that hold a column twice: two lanes of one step meet
-    A, B = _narrow(40, 700, 40, 9, repeat=True)
+    A, B = _narrow(1100, 700, 40, 9, repeat=True)
     C, st = multiply_device(A, B, {"force_workflow": wf})
     check(A, B, C)
     assert st["decision"]["workflow"] == wf
