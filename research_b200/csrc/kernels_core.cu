@@ -1251,7 +1251,7 @@ __device__ __forceinline__ void mark_bit(unsigned long long* bits, uint32_t c, b
 // slots (one per column) takes the place of an atomic, and there is no block
 // barrier and no owner search. Four entries' loads are in flight. 2 * 10^5
 // banded rows (256/64, 7.2 * 10^8 products), one B200, block kernels -> these:
-// symbolic 1.9 -> 0.80 ms, numeric 4.4 -> 2.3 ms (315 G products/s; 20 warps
+// symbolic 1.9 -> 0.8 ms, numeric 4.4 -> 2.2 ms (330 G products/s; 20 warps
 // per SM by the slots, so the loads' latency is what is left); dense blocks
 // 256/64 of 57 entries a row, numeric 1.88 -> 1.3 ms.
 // op(column offset, value, same) for the products of A entries [a0, a1), by the
@@ -1339,21 +1339,33 @@ __global__ void __launch_bounds__(kNarrowWarps * 32)
   __syncwarp();
   unsigned mine = 0;
   const uint32_t count = *q.count;
-  for (uint64_t idx = (uint64_t)blockIdx.x * kNarrowWarps + warp; idx < count; idx += (uint64_t)gridDim.x * kNarrowWarps) {
-    const uint32_t row = q.rows[idx];
-    const uint32_t rlo = lo[row], span1 = hi[row] - rlo;
-    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
-    if (!narrow_row(prod[row], a1 - a0, (uint64_t)span1 + 1, kNarrowSym)) continue;
-    warp_for_each_product<false>(A, B, a0, a1, rlo, span1, [&](uint32_t d, double, bool) { flag[d] = 1; });
-    uint32_t n = 0;
-    for (uint32_t i = lane; i <= span1 >> 2; i += 32) {
-      n += __popc(words[i]);
-      words[i] = 0u;
+  // the warp's next 32 rows are looked at together, a lane each (a list of 2^18
+  // rows without a narrow one, row by row: 0.25 ms)
+  const uint64_t warps = (uint64_t)gridDim.x * kNarrowWarps;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * kNarrowWarps + warp; i0 < count; i0 += 32 * warps) {
+    const uint64_t ahead = i0 + lane * warps;
+    uint32_t my_row = 0;
+    bool take = false;
+    if (ahead < count) {
+      my_row = q.rows[ahead];
+      take = narrow_row(prod[my_row], A.row_end(my_row) - A.row_begin(my_row),
+                        (uint64_t)hi[my_row] - lo[my_row] + 1, kNarrowSym);
     }
-    n = __reduce_add_sync(kFull, n);
-    if (lane == 0) row_nnz[row] = n;
-    ++mine;
-    __syncwarp();
+    for (unsigned todo = __ballot_sync(kFull, take); todo; todo &= todo - 1) {
+      const uint32_t row = __shfl_sync(kFull, my_row, __ffs(todo) - 1);
+      const uint32_t rlo = lo[row], span1 = hi[row] - rlo;
+      const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+      warp_for_each_product<false>(A, B, a0, a1, rlo, span1, [&](uint32_t d, double, bool) { flag[d] = 1; });
+      uint32_t n = 0;
+      for (uint32_t i = lane; i <= span1 >> 2; i += 32) {
+        n += __popc(words[i]);
+        words[i] = 0u;
+      }
+      n = __reduce_add_sync(kFull, n);
+      if (lane == 0) row_nnz[row] = n;
+      ++mine;
+      __syncwarp();
+    }
   }
   if (lane == 0 && mine) atomicAdd(done, mine);
 }
@@ -1376,46 +1388,58 @@ __global__ void __launch_bounds__(kNarrowWarps * 32)
   __syncwarp();
   unsigned mine = 0;
   const uint32_t count = *q.count;
-  for (uint64_t idx = (uint64_t)blockIdx.x * kNarrowWarps + warp; idx < count; idx += (uint64_t)gridDim.x * kNarrowWarps) {
-    const uint32_t row = q.rows[idx];
-    const uint32_t rlo = lo[row], span1 = hi[row] - rlo;
-    const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
-    if (!narrow_row(prod[row], a1 - a0, (uint64_t)span1 + 1, kNarrowNum)) continue;
-    warp_for_each_product<true>(A, B, a0, a1, rlo, span1, [&](uint32_t d, double v, bool same) {
-      if (same) atomicAdd(&acc[d], v);
-      else acc[d] += v;
-      flag[d] = 1;
-    });
-    const uint32_t cap = o.cap[row];
-    const uint64_t off = o.off[row];
-    uint32_t lim = cap;
-    if (o.count) {  // estimated slots: the count decides whether the row is written
-      uint32_t n = 0;
-      for (uint32_t i = lane; i <= span1; i += 32) n += flag[i];
-      n = __reduce_add_sync(kFull, n);
-      int accept = 0;
-      if (lane == 0) accept = out_accept(o, ctr, row, n, cap);
-      if (!__shfl_sync(kFull, accept, 0)) lim = 0;
+  // the warp's next 32 rows are looked at together, a lane each (a list of 2^18
+  // rows without a narrow one, row by row: 0.25 ms)
+  const uint64_t warps = (uint64_t)gridDim.x * kNarrowWarps;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * kNarrowWarps + warp; i0 < count; i0 += 32 * warps) {
+    const uint64_t ahead = i0 + lane * warps;
+    uint32_t my_row = 0;
+    bool take = false;
+    if (ahead < count) {
+      my_row = q.rows[ahead];
+      take = narrow_row(prod[my_row], A.row_end(my_row) - A.row_begin(my_row),
+                        (uint64_t)hi[my_row] - lo[my_row] + 1, kNarrowNum);
     }
-    uint32_t at = 0;
-    for (uint32_t i0 = 0; i0 <= span1; i0 += 32) {
-      const uint32_t i = i0 + lane;  // (the slots are a multiple of 32)
-      const bool f = flag[i] != 0;
-      const unsigned m = __ballot_sync(kFull, f);
-      if (f) {
-        const uint32_t w = at + __popc(m & lt);
-        if (w < lim) {
-          c_col[off + w] = rlo + i;
-          c_val[off + w] = acc[i];
-        }
-        acc[i] = 0.0;
-        flag[i] = 0;
+    for (unsigned todo = __ballot_sync(kFull, take); todo; todo &= todo - 1) {
+      const uint32_t row = __shfl_sync(kFull, my_row, __ffs(todo) - 1);
+      const uint32_t rlo = lo[row], span1 = hi[row] - rlo;
+      const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
+      warp_for_each_product<true>(A, B, a0, a1, rlo, span1, [&](uint32_t d, double v, bool same) {
+        if (same) atomicAdd(&acc[d], v);
+        else acc[d] += v;
+        flag[d] = 1;
+      });
+      const uint32_t cap = o.cap[row];
+      const uint64_t off = o.off[row];
+      uint32_t lim = cap;
+      if (o.count) {  // estimated slots: the count decides whether the row is written
+        uint32_t n = 0;
+        for (uint32_t i = lane; i <= span1; i += 32) n += flag[i];
+        n = __reduce_add_sync(kFull, n);
+        int accept = 0;
+        if (lane == 0) accept = out_accept(o, ctr, row, n, cap);
+        if (!__shfl_sync(kFull, accept, 0)) lim = 0;
       }
-      at += __popc(m);
+      uint32_t at = 0;
+      for (uint32_t i0 = 0; i0 <= span1; i0 += 32) {
+        const uint32_t i = i0 + lane;  // (the slots are a multiple of 32)
+        const bool f = flag[i] != 0;
+        const unsigned m = __ballot_sync(kFull, f);
+        if (f) {
+          const uint32_t w = at + __popc(m & lt);
+          if (w < lim) {
+            c_col[off + w] = rlo + i;
+            c_val[off + w] = acc[i];
+          }
+          acc[i] = 0.0;
+          flag[i] = 0;
+        }
+        at += __popc(m);
+      }
+      if (!o.count && lane == 0) out_accept(o, ctr, row, at, cap);
+      ++mine;
+      __syncwarp();
     }
-    if (!o.count && lane == 0) out_accept(o, ctr, row, at, cap);
-    ++mine;
-    __syncwarp();
   }
   if (lane == 0 && mine) atomicAdd(done, mine);
 }
