@@ -2744,7 +2744,7 @@ struct WinItem {
 
 // One block per row: popcounts of the groups, then one thread cuts them into
 // items. The other rows go to the rest list.
-__global__ void __launch_bounds__(256) k_item_plan(RowQueue q, const DevCounters* __restrict__ ctr,
+__global__ void __launch_bounds__(256) k_item_plan(RowQueue q, DevCounters* __restrict__ ctr,
                                                    unsigned long long shares, const uint32_t* __restrict__ prod,
                                                    const uint32_t* __restrict__ lo,
                                                    const uint32_t* __restrict__ hi,
@@ -2758,6 +2758,7 @@ __global__ void __launch_bounds__(256) k_item_plan(RowQueue q, const DevCounters
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t count = *q.count;
   const unsigned long long heavy = ctr->num_prod[NB_BITMAP] / shares;
+  uint32_t my_rows = 0, my_items = 0;  // thread 0: what this block has cut
   for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
     const uint32_t row = q.rows[idx];
     const uint64_t slot = bm_off[row];
@@ -2793,6 +2794,8 @@ __global__ void __launch_bounds__(256) k_item_plan(RowQueue q, const DevCounters
         rest[atomicAdd(&ic->rest, 1u)] = row;
         s_n = 0;
       }
+      my_rows += s_n != 0;
+      my_items += s_n;
     }
     __syncthreads();
     // a warp per item: its rank is the popcount of the groups before it
@@ -2808,6 +2811,10 @@ __global__ void __launch_bounds__(256) k_item_plan(RowQueue q, const DevCounters
       if (lane == 0) items[s_base + i] = WinItem{row, g0, g1, before, n};
     }
     __syncthreads();
+  }
+  if (threadIdx.x == 0 && my_rows) {
+    atomicAdd(&ctr->item_rows, my_rows);
+    atomicAdd(&ctr->item_count, my_items);
   }
 }
 

@@ -92,7 +92,11 @@ struct Stats {
   uint64_t sym_prod[SB_COUNT] = {0};
   uint64_t cache_words = 0, cache_used = 0;
   bool cache_dropped = false;
-  int bm_kernel = 0;  // numeric bitmap class: 0 no rows, 1 k_num_bitmap (rank + FP64 red), 2 k_num_window
+  // numeric bitmap class: 0 no rows, 1 k_num_bitmap (rank + FP64 red; the rows counted in item_rows in
+  // k_num_items), 2 k_num_window
+  int bm_kernel = 0;
+  uint64_t item_rows = 0, items = 0;            // bitmap rows cut into window items, and their items
+  uint64_t sym_narrow_rows = 0, num_narrow_rows = 0;  // rows of the narrow-row kernels
   int host_chunks = 0;  // host-buffer multiply: row chunks whose copies overlapped the numeric phase (0: none)
   bool fused = false;  // ultra-sparse workflow in one fused launch
   int launches = 0;  // kernels launched by the last call
@@ -1251,6 +1255,10 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
   st.max_a_nnz = h->h_ctr->max_a_nnz;
   for (int i = 0; i < SB_COUNT; ++i) st.sym_bins[i] = h->h_ctr->sym_count[i];
   for (int i = 0; i < NB_COUNT; ++i) st.num_bins[i] = h->h_ctr->num_count[i];
+  st.item_rows = h->h_ctr->item_rows;
+  st.items = h->h_ctr->item_count;
+  for (int i = 0; i < SB_COUNT; ++i) st.sym_narrow_rows += h->h_ctr->sym_narrow_done[i];
+  for (int i = 0; i < NB_COUNT; ++i) st.num_narrow_rows += h->h_ctr->num_narrow_done[i];
   for (int i = 0; i < NB_COUNT; ++i) {
     st.num_nnz[i] = h->h_ctr->num_nnz[i];
     st.num_anz[i] = h->h_ctr->num_anz[i];
@@ -1329,7 +1337,9 @@ std::string stats_json(ocean_handle* h) {
     << ", \"bitmap_cache_dropped\": " << (st.cache_dropped ? "true" : "false")
     << ", \"fused_ultrasparse\": " << (st.fused ? "true" : "false")
     << ", \"numeric_bitmap_kernel\": \"" << (st.bm_kernel == 2 ? "window" : st.bm_kernel == 1 ? "rank" : "none")
-    << "\", \"host_pipeline_chunks\": " << st.host_chunks << ", \"kernel_launches\": " << st.launches << "}, ";
+    << "\", \"window_item_rows\": " << st.item_rows << ", \"window_items\": " << st.items
+    << ", \"symbolic_narrow_rows\": " << st.sym_narrow_rows
+    << ", \"numeric_narrow_rows\": " << st.num_narrow_rows << ", \"host_pipeline_chunks\": " << st.host_chunks << ", \"kernel_launches\": " << st.launches << "}, ";
   if (st.sampled)
     o << "\"sampling\": {\"compaction_1\": " << st.compaction1 << ", \"compaction_2\": " << st.compaction2
       << "}, ";

@@ -76,6 +76,8 @@ struct DevCounters {
   unsigned int num_narrow;   // the numeric hash classes have rows for k_num_narrow
   unsigned int sym_narrow_done[SB_COUNT];  // rows of each class that k_sym_narrow has counted
   unsigned int num_narrow_done[NB_COUNT];  // rows of each class that k_num_narrow has written
+  unsigned int item_rows;    // numeric bitmap-class rows cut into window items
+  unsigned int item_count;   // their window items
 };
 
 // Rows of A with more than kLongRowEntries entries are not summarised by one

@@ -30,6 +30,10 @@ def test_power_law_rows(cols, wide_pointers):
     check(A, B, C)
     assert st["decision"]["bitmap_cache_used_bytes"] > 0
     assert int(np.diff(C.rowptr.astype(np.int64)).max()) > 20480  # rows of several items
+    d = st["decision"]
+    assert 0 < d["window_item_rows"] < d["window_items"]
+    if cols <= 1 << 18:  # every row with a saved bitmap
+        assert d["window_item_rows"] == st["binning_1"][SYM_BINS["bitmap"]]
 
 
 @pytest.mark.parametrize("span", [64, 2048, 2049, 1 << 18, (1 << 19) + 1, 1 << 20])
@@ -67,4 +71,5 @@ def test_items_in_the_host_pipeline(chunks):
     g = SpGEMM({"host_pipeline_chunks": chunks, "host_pipeline_min_products": 1, "small_problem_nnz": 0})
     C = g.multiply(A, B)
     check(A, B, C)
-    assert g.get_stats()["decision"]["host_pipeline_chunks"] == chunks
+    d = g.get_stats()["decision"]
+    assert d["host_pipeline_chunks"] == chunks and d["window_item_rows"] > 0
