@@ -1460,8 +1460,13 @@ struct SymHashSmem {
   uint32_t s_idx;
 };
 
+// As many blocks per SM as the shared memory allows (16, 5 and 1): left to
+// itself the compiler took 40 to 48 registers for the blocks of 128 threads (12
+// or 10 per SM), and the hashed rows wait on their shared-memory probes (2^18
+// uniform rows of 32 entries, this class: 10 blocks 2.01 ms, 12 1.85, 16 1.76;
+// marked rows of a 16-entry band 208 and 173 us at 12 and 16).
 template <typename RP, int NT, int LOG2T>
-__global__ void __launch_bounds__(NT) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue q, DevCounters* __restrict__ ctr,
+__global__ void __launch_bounds__(NT, NT == 128 ? 16 : NT == 256 ? 5 : 1) k_sym_hash(Csr<RP> A, Csr<RP> B, RowQueue q, DevCounters* __restrict__ ctr,
                                                  const uint32_t* __restrict__ prod, const uint32_t* __restrict__ maxb,
                                                  const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
                                                  uint32_t* __restrict__ row_nnz, NarrowDone narrow) {
