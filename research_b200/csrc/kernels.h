@@ -65,10 +65,9 @@ struct DevWork {
   uint32_t* chunk_bound = nullptr;
   unsigned* chunk_count = nullptr;
   unsigned* chunk_cursor = nullptr;
-  // symbolic hash classes (bits) that may have narrow rows, and whether the
-  // numeric ones have any (0: the narrow-row kernels are not launched and every
-  // row runs in its class kernel)
-  unsigned sym_narrow = 0, num_narrow = 0;
+  // most lane slots of a narrow row of each class (0: the narrow-row kernel is
+  // not launched and every row runs in its class kernel)
+  uint32_t sym_narrow[SB_COUNT] = {0}, num_narrow[NB_COUNT] = {0};
   // segment-driven dispatch: per-row policy slot (0: the call's policy,
   // 1 + SegClass: that segment class's policy); null: slot 0 for every row
   const uint8_t* row_pol = nullptr;
@@ -215,12 +214,17 @@ int launch_row_bounds(const DevWork& w, uint32_t* out, cudaStream_t s);
 void configure_kernel_attributes();
 bool ensure_kernel_attributes(int dev);
 
-// Symbolic hash classes (bits) whose list k_sym_narrow looks through before the
-// class kernel: at least 1024 rows, whose B rows have 8 entries and more in the
-// mean. Decided from the class sums: a test of every row in the analysis cost
-// the row sizing of the 2^21 power-law graph 9 us of 2265, a look through the
-// list of 2^18 rows without a narrow one costs less than 0.2 ms of 7.7.
-unsigned sym_narrow_classes(const DevCounters& c);
+// Limits of the narrow rows (DevWork::sym_narrow) from the counters read back
+// after the analysis: classes of at least 1024 rows, whose B rows have 8 entries
+// and more in the mean. Decided from the class sums: a test of every row in the
+// analysis cost the row sizing of the 2^21 power-law graph 9 us of 2265, a look
+// through the list of 2^18 rows without a narrow one costs less than 0.2 ms of 7.7.
+// Null: no narrow rows.
+void set_sym_narrow(DevWork& w, const DevCounters* c, int num_sms);
+// The same for the numeric classes, from the sums over their narrow rows that
+// the scan made; null: not known, no narrow rows. chunks: row chunks of equal
+// products that the numeric phase runs in (0: none).
+void set_num_narrow(DevWork& w, const DevCounters* c, int num_sms, int chunks = 0);
 
 // Most window items of `rows` bitmap-class rows with `nnz` output entries, and
 // the bytes of one.

@@ -133,10 +133,32 @@ __device__ __forceinline__ uint32_t spread_index(uint32_t idx, uint32_t count, u
 // multiply, in their block class -> a warp each: bands of 12 entries a row
 // 664 -> 530 us, 16 entries 968 -> 569 us, 24 entries 1334 -> 713 us; blocks of
 // 16 entries 946 -> 553 us, 32 entries 951 -> 942 us).
+// `limit` bounds the lane slots of such a row (narrow_slots; see narrow_limit).
 constexpr uint32_t kNarrowSym = 4096;  // columns of a symbolic row
 constexpr uint32_t kNarrowNum = 1088;  // columns of a numeric row: 9.6 KB a warp, 20 warps per SM
-__device__ __forceinline__ bool narrow_row(uint64_t p, uint64_t anz, uint64_t span, uint32_t most) {
-  return span <= most && p > 128 && p >= 8 * anz;
+// Lane slots of a row in the steps of one warp: its products, and half a step
+// lost per A entry.
+__host__ __device__ __forceinline__ uint64_t narrow_slots(uint64_t p, uint64_t anz) { return p + 16 * anz; }
+__device__ __forceinline__ bool narrow_row(uint64_t p, uint64_t anz, uint64_t span, uint32_t most, uint32_t limit) {
+  return span <= most && p > 128 && p >= 8 * anz && narrow_slots(p, anz) <= limit;
+}
+// Most lane slots of a narrow row where the narrow rows of a class are `rows`
+// with `products` and `anz` A entries in all, 0: none of them runs a warp each.
+// A warp by itself walks 0.18 slots a ns and the block kernels 165 products a ns
+// on the whole GPU, so a row of more than products / 917 slots is still under way
+// when the block kernels would be done with all rows. The class is left to them
+// when its mean row has more than 1.25 times that (products / (5 SMs): few rows,
+// or heavy ones), or when that is below 512 slots (a few microseconds of work);
+// otherwise the rows of more than 1.5 times the mean allowed are, so that nearly
+// equal rows are not split over two launches. Whole multiplies, one B200, every
+// narrow row a warp -> by this rule: power-law 2^10 rows of 16 entries 342 -> 239
+// us; 3 rows of 320000 products 3.93 -> 0.88 ms; 600 rows of 16000 products, B
+// rows of 16 entries, 1068 -> 899 us (1500 such rows stay narrow: 1078 us); 1000
+// rows of a 64-entry band 197 -> 181 us (1400 stay narrow: 197 us).
+static uint32_t narrow_limit(uint64_t rows, uint64_t products, uint64_t anz, int num_sms) {
+  const uint64_t most = products / (5ull * num_sms);
+  if (most < 512 || narrow_slots(products, anz) > most * rows) return 0;
+  return (uint32_t)std::min<uint64_t>(most + most / 2, 0xFFFFFFFFu);
 }
 
 // ---------------------------------------------------------------- analysis
@@ -1316,21 +1338,21 @@ __device__ __forceinline__ void warp_for_each_product(const Csr<RP>& A, const Cs
 
 constexpr int kNarrowWarps = 4;
 
-// What a class kernel knows of the narrow rows of its list: on, they are
-// skipped; when `done` counts the whole list, there is nothing else in it (a
+// What a class kernel knows of the narrow rows of its list: with a limit, they
+// are skipped; when `done` counts the whole list, there is nothing else in it (a
 // list of 2 * 10^5 skipped rows costs a class kernel 0.3 ms). `done` is null
 // where a list is one of several row chunks.
 struct NarrowDone {
-  bool on;
+  uint32_t limit;
   const unsigned* done;
-  __device__ bool all(uint32_t count) const { return on && done && *done == count; }
+  __device__ bool all(uint32_t count) const { return limit && done && *done == count; }
 };
 
 template <typename RP>
 __global__ void __launch_bounds__(kNarrowWarps * 32)
     k_sym_narrow(Csr<RP> A, Csr<RP> B, RowQueue q, const uint32_t* __restrict__ prod,
                  const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi, uint32_t* __restrict__ row_nnz,
-                 unsigned* __restrict__ done) {
+                 uint32_t limit, unsigned* __restrict__ done) {
   __shared__ __align__(16) uint8_t s_flag[kNarrowWarps][kNarrowSym];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* flag = s_flag[warp];
@@ -1349,7 +1371,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32)
     if (ahead < count) {
       my_row = q.rows[ahead];
       take = narrow_row(prod[my_row], A.row_end(my_row) - A.row_begin(my_row),
-                        (uint64_t)hi[my_row] - lo[my_row] + 1, kNarrowSym);
+                        (uint64_t)hi[my_row] - lo[my_row] + 1, kNarrowSym, limit);
     }
     for (unsigned todo = __ballot_sync(kFull, take); todo; todo &= todo - 1) {
       const uint32_t row = __shfl_sync(kFull, my_row, __ffs(todo) - 1);
@@ -1374,7 +1396,8 @@ template <typename RP>
 __global__ void __launch_bounds__(kNarrowWarps * 32)
     k_num_narrow(Csr<RP> A, Csr<RP> B, RowQueue q, OutSpec o, DevCounters* __restrict__ ctr,
                  const uint32_t* __restrict__ prod, const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi,
-                 uint32_t* __restrict__ c_col, double* __restrict__ c_val, unsigned* __restrict__ done) {
+                 uint32_t* __restrict__ c_col, double* __restrict__ c_val, uint32_t limit,
+                 unsigned* __restrict__ done) {
   __shared__ double s_acc[kNarrowWarps][kNarrowNum];
   __shared__ uint8_t s_flag[kNarrowWarps][kNarrowNum];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1398,7 +1421,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32)
     if (ahead < count) {
       my_row = q.rows[ahead];
       take = narrow_row(prod[my_row], A.row_end(my_row) - A.row_begin(my_row),
-                        (uint64_t)hi[my_row] - lo[my_row] + 1, kNarrowNum);
+                        (uint64_t)hi[my_row] - lo[my_row] + 1, kNarrowNum, limit);
     }
     for (unsigned todo = __ballot_sync(kFull, take); todo; todo &= todo - 1) {
       const uint32_t row = __shfl_sync(kFull, my_row, __ffs(todo) - 1);
@@ -1487,7 +1510,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 16 : NT == 256 ? 5 : 1) k_sym_
     const uint32_t span1 = hi[row] - rlo;
     const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
     const uint32_t np = prod[row];
-    if (narrow.on && narrow_row(np, a1 - a0, (uint64_t)span1 + 1, kNarrowSym)) {  // k_sym_narrow's rows
+    if (narrow.limit && narrow_row(np, a1 - a0, (uint64_t)span1 + 1, kNarrowSym, narrow.limit)) {  // k_sym_narrow's rows
       __syncthreads();
       continue;
     }
@@ -1634,7 +1657,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B
     const uint32_t cap = o.cap[row];
     const uint64_t off = o.off[row];
     if (span1 >= (uint32_t)kBitmapBits ||  // k_num_hash's rows
-        (narrow.on && narrow_row(np, a1 - a0, (uint64_t)span1 + 1, kNarrowNum))) {  // k_num_narrow's rows
+        (narrow.limit && narrow_row(np, a1 - a0, (uint64_t)span1 + 1, kNarrowNum, narrow.limit))) {  // k_num_narrow's rows
       __syncthreads();
       continue;
     }
@@ -3142,11 +3165,11 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
                                                      const uint32_t* __restrict__ chunk_bound,
                                                      unsigned* __restrict__ chunk_count) {
   __shared__ unsigned long long scr[33];
-  __shared__ unsigned long long s_cls[3][NB_COUNT];
+  __shared__ unsigned long long s_cls[6][NB_COUNT];
   __shared__ unsigned s_cnt[NB_COUNT * kMaxChunks];
   __shared__ uint32_t s_bound[kMaxChunks + 1];
   const int nseg = chunks > 1 ? chunks : 1;
-  if (threadIdx.x < 3 * NB_COUNT) (&s_cls[0][0])[threadIdx.x] = 0ull;
+  if (threadIdx.x < 6 * NB_COUNT) (&s_cls[0][0])[threadIdx.x] = 0ull;
   if (threadIdx.x < NB_COUNT * kMaxChunks) s_cnt[threadIdx.x] = 0u;
   if (nseg > 1 && (int)threadIdx.x <= nseg) s_bound[threadIdx.x] = chunk_bound[threadIdx.x];
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * 4;
@@ -3175,8 +3198,10 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
   }
   int bq[4], sq[4];
   uint32_t rq[4], aq[4], pq[4];
+  bool nq[4];  // narrow rows, whatever their limit
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
+    nq[q] = false;
     const uint64_t i = base + q;
     int b = -1;
     if (i < n) {
@@ -3192,9 +3217,8 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       if (b == NB_BITMAP && (uint64_t)hi[i] - lo[i] + 1 > kBitmapBits) atomicAdd(&ctr->num_wide, 1u);
       aq[q] = anz[i];
       pq[q] = p;
-      if ((b == NB_HASH_S || b == NB_HASH_M) && pols.p[0].force_bin < 0 &&
-          narrow_row(p, aq[q], (uint64_t)hi[i] - lo[i] + 1, kNarrowNum))
-        ctr->num_narrow = 1u;
+      nq[q] = (b == NB_HASH_S || b == NB_HASH_M) && pols.p[0].force_bin < 0 &&
+              narrow_row(p, aq[q], (uint64_t)hi[i] - lo[i] + 1, kNarrowNum, 0xFFFFFFFFu);
     }
     bq[q] = b;
     rq[q] = (uint32_t)i;
@@ -3235,12 +3259,40 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       atomicAdd(&s_cls[1][c], b2);
       atomicAdd(&s_cls[2][c], d);
     }
+    // the class's narrow rows
+    bool any = false;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) any |= bq[q] == c && nq[q];
+    if (__any_sync(kFull, any)) {
+      unsigned long long r = 0, e = 0, f = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (bq[q] == c && nq[q]) {
+          ++r;
+          e += aq[q];
+          f += pq[q];
+        }
+      }
+      r = warp_sum_u64(r);
+      e = warp_sum_u64(e);
+      f = warp_sum_u64(f);
+      if (lane == 0) {
+        atomicAdd(&s_cls[3][c], r);
+        atomicAdd(&s_cls[4][c], e);
+        atomicAdd(&s_cls[5][c], f);
+      }
+    }
   }
   __syncthreads();
   if (threadIdx.x < NB_COUNT && s_cls[0][threadIdx.x]) {
     atomicAdd(&ctr->num_nnz[threadIdx.x], s_cls[0][threadIdx.x]);
     atomicAdd(&ctr->num_anz[threadIdx.x], s_cls[1][threadIdx.x]);
     atomicAdd(&ctr->num_prod[threadIdx.x], s_cls[2][threadIdx.x]);
+    if (s_cls[3][threadIdx.x]) {
+      atomicAdd(&ctr->narrow_rows[threadIdx.x], s_cls[3][threadIdx.x]);
+      atomicAdd(&ctr->narrow_anz[threadIdx.x], s_cls[4][threadIdx.x]);
+      atomicAdd(&ctr->narrow_prod[threadIdx.x], s_cls[5][threadIdx.x]);
+    }
   }
 }
 
@@ -3640,11 +3692,20 @@ bool ensure_kernel_attributes(int dev) {
 uint64_t item_capacity(uint64_t rows, uint64_t nnz) { return nnz / (kItemV - 2048) + 3 * rows + 1; }
 size_t item_bytes() { return sizeof(WinItem); }
 
-unsigned sym_narrow_classes(const DevCounters& c) {
-  unsigned mask = 0;
-  for (int k = SB_HASH_S; k <= SB_HASH_L; ++k)
-    if (c.sym_count[k] >= 1024 && c.sym_prod[k] >= 8 * c.sym_anz[k]) mask |= 1u << k;
-  return mask;
+void set_sym_narrow(DevWork& w, const DevCounters* c, int num_sms) {
+  for (int k = 0; k < SB_COUNT; ++k) {
+    const bool hash = c && k >= SB_HASH_S && k <= SB_HASH_L;
+    w.sym_narrow[k] = hash && c->sym_count[k] >= 1024 && c->sym_prod[k] >= 8 * c->sym_anz[k]
+                          ? narrow_limit(c->sym_count[k], c->sym_prod[k], c->sym_anz[k], num_sms)
+                          : 0u;
+  }
+}
+
+void set_num_narrow(DevWork& w, const DevCounters* c, int num_sms, int chunks) {
+  const uint64_t d = chunks > 1 ? chunks : 1;
+  for (int k = 0; k < NB_COUNT; ++k)
+    w.num_narrow[k] =
+        c ? narrow_limit(c->narrow_rows[k] / d, c->narrow_prod[k] / d, c->narrow_anz[k] / d, num_sms) : 0u;
 }
 
 size_t window_scratch_words(int num_sms) { return (size_t)num_sms * (size_t)g_occ[K_NUM_WIN] * kBitmapWords; }
@@ -3725,12 +3786,13 @@ int launch_symbolic(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, int nu
     k_sym_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(SB_ESC4), w.ctr, w.row_nnz);
   // narrow rows of the hash classes, a warp each (timed with the small-hash class)
   auto narrow_done = [&](int cls) {
-    return NarrowDone{((w.sym_narrow >> cls) & 1u) != 0, w.ctr->sym_narrow_done + cls};
+    return NarrowDone{w.sym_narrow[cls], w.ctr->sym_narrow_done + cls};
   };
   auto narrow = [&](int cls) {
-    if (((w.sym_narrow >> cls) & 1u) && ++launched)
-      k_sym_narrow<RP><<<9 * num_sms, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), w.prod, w.lo, w.hi, w.row_nnz,
-                                                                  w.ctr->sym_narrow_done + cls);
+    const unsigned g = w.sym_narrow[cls] ? class_grid(num_sms, 9, counts, cls, kNarrowWarps) : 0u;
+    if (g && ++launched)
+      k_sym_narrow<RP><<<g, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), w.prod, w.lo, w.hi, w.row_nnz,
+                                                       w.sym_narrow[cls], w.ctr->sym_narrow_done + cls);
   };
   mark(SB_HASH_S);
   narrow(SB_HASH_S);
@@ -3835,12 +3897,13 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
   if ((gsz = grid(K_NUM_ESC4, NB_ESC4, 8)) && ++launched)
     k_num_esc<RP, 4><<<gsz, 256, 0, s>>>(A, B, queue(NB_ESC4), o, w.ctr, c_col, c_val);
   auto narrow_done = [&](int cls) {
-    return NarrowDone{w.num_narrow != 0, chunked ? nullptr : w.ctr->num_narrow_done + cls};
+    return NarrowDone{w.num_narrow[cls], chunked ? nullptr : w.ctr->num_narrow_done + cls};
   };
   auto narrow = [&](int cls) {
-    if (w.num_narrow && (!counts || counts[cls]) && ++launched)
-      k_num_narrow<RP><<<5 * num_sms, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), o, w.ctr, w.prod, w.lo, w.hi, c_col,
-                                                                 c_val, w.ctr->num_narrow_done + cls);
+    const unsigned g = w.num_narrow[cls] ? class_grid(num_sms, 5, counts, cls, kNarrowWarps) : 0u;
+    if (g && ++launched)
+      k_num_narrow<RP><<<g, kNarrowWarps * 32, 0, s>>>(A, B, queue(cls), o, w.ctr, w.prod, w.lo, w.hi, c_col, c_val,
+                                                       w.num_narrow[cls], w.ctr->num_narrow_done + cls);
   };
   mark(NB_HASH_S);
   narrow(NB_HASH_S);
@@ -3864,7 +3927,7 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
   if ((gsz = grid(K_NUM_L, NB_HASH_L, 1)) && ++launched)
     k_num_rank<RP, 512, 4096><<<gsz, 512, num_rank_smem<512, 4096>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.prod, w.maxb,
                                                                   w.lo, w.hi, c_col, c_val,
-                                                                  NarrowDone{false, nullptr});
+                                                                  NarrowDone{0u, nullptr});
   if (wide && gsz && ++launched)
     k_num_hash<RP, 512, 13><<<gsz, 512, num_hash_smem<512, 13>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.lo, w.hi,
                                                                   c_col, c_val);

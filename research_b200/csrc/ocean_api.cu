@@ -726,7 +726,7 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
       }
     }
   }
-  h->w.sym_narrow = h->cfg.force_sym_bin < 0 ? sym_narrow_classes(*h->h_ctr) : 0u;
+  set_sym_narrow(h->w, h->cfg.force_sym_bin < 0 ? h->h_ctr : nullptr, h->num_sms);
   // per-class boundary events only when stage timing is asked for (each record costs device time)
   const bool track = h->cfg.track_stage_times;
   h->st.launches += launch_symbolic(A, B, h->w, h->num_sms, s, track ? h->ev + EV_SYM0 : nullptr,
@@ -1148,7 +1148,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         for (int i = 0; i < NB_COUNT; ++i) num_counts[i] = h->h_ctr->num_count[i];
         const OutSpec est_out{h->w.est_off, h->w.est, h->w.cnt, h->w.ovf, &h->w.ctr->overflow_n};
         st.bm_kernel = num_counts[NB_BITMAP] ? 1 : 0;
-        h->w.num_narrow = class_counts ? h->h_ctr->num_narrow : 0u;
+        set_num_narrow(h->w, class_counts ? h->h_ctr : nullptr, h->num_sms);
         st.launches += launch_numeric(A, B, h->w, est_out, (uint32_t*)t_col, (double*)t_val, h->num_sms, s,
                                       track ? h->ev + EV_NUM0 : nullptr, class_counts ? num_counts : nullptr);
         if (track) h->ev_mask |= ((1ull << (NB_COUNT + 1)) - 1) << EV_NUM0;
@@ -1190,7 +1190,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         for (int i = 0; i < NB_COUNT; ++i) num_counts[i] = h->h_ctr->num_count[i];
         prepare_windows(h, A.nnz, num_counts[NB_BITMAP]);
         prepare_items(h, num_counts[NB_BITMAP], h->h_ctr->num_nnz[NB_BITMAP]);
-        h->w.num_narrow = h->h_ctr->num_narrow;
+        set_num_narrow(h->w, h->h_ctr, h->num_sms, h->w.chunks);
         const OutSpec exact{h->w.rowptr64, h->w.row_nnz, nullptr, nullptr, nullptr};
         if (h->w.chunks) {
           st.launches += pipeline_numeric(h, A, B, exact, owner, nnz, bits, s);
@@ -1600,7 +1600,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
     batch_readback(b, s);
     const DevCounters& k = *b->h_ctr;
     for (int i = 0; i < SB_COUNT; ++i) b->sym_counts[i] = k.sym_count[i];
-    w.sym_narrow = b->cfg.force_sym_bin < 0 ? sym_narrow_classes(k) : 0u;
+    set_sym_narrow(w, b->cfg.force_sym_bin < 0 ? &k : nullptr, h->num_sms);
     b->products = k.total_products;
     const Config& c = b->cfg;
     const double avg = A.rows ? (double)k.total_products / (double)A.rows : 0.0;
@@ -1626,7 +1626,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
       batch_readback(b, s);
       b->c_nnz = b->h_ctr->total_nnz;
       for (int i = 0; i < NB_COUNT; ++i) b->num_counts[i] = b->h_ctr->num_count[i];
-      w.num_narrow = b->h_ctr->num_narrow;
+      set_num_narrow(w, b->h_ctr, h->num_sms);
     } else {
       launch_batch_guard(w.ctr, &w.ctr->total_nnz, b->c_nnz, s);
       launched += 1;
@@ -1652,7 +1652,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
       batch_readback(b, s);
       b->total_est = b->h_ctr->total_est;
       for (int i = 0; i < NB_COUNT; ++i) b->num_counts[i] = b->h_ctr->num_count[i];
-      w.num_narrow = b->h_ctr->num_narrow;
+      set_num_narrow(w, b->h_ctr, h->num_sms);
       OCEAN_CUDA(cudaMalloc((void**)&b->t_col, std::max<uint64_t>(b->total_est, 1) * 4));
       OCEAN_CUDA(cudaMalloc((void**)&b->t_val, std::max<uint64_t>(b->total_est, 1) * 8));
     } else {

@@ -73,7 +73,9 @@ struct DevCounters {
   unsigned int num_long;     // rows of A listed as long (more than kLongRowEntries entries)
   unsigned int long_chunks;  // chunks of kLongChunk A entries of the listed rows
   unsigned int pad[1];
-  unsigned int num_narrow;   // the numeric hash classes have rows for k_num_narrow
+  unsigned long long narrow_rows[NB_COUNT];  // narrow rows of each numeric class, whatever their limit,
+  unsigned long long narrow_anz[NB_COUNT];   // their A entries
+  unsigned long long narrow_prod[NB_COUNT];  // and products
   unsigned int sym_narrow_done[SB_COUNT];  // rows of each class that k_sym_narrow has counted
   unsigned int num_narrow_done[NB_COUNT];  // rows of each class that k_num_narrow has written
   unsigned int item_rows;    // numeric bitmap-class rows cut into window items

@@ -84,6 +84,16 @@ def test_chunked_rectangular():
     check(A, B, C)
 
 
+@pytest.mark.parametrize("chunks", [2, 5])
+def test_chunked_narrow_rows(chunks):
+    # bands whose rows run a warp each, in every chunk's class lists
+    A = M.banded(30000, 100, 24, seed=6)
+    C, st = host_multiply(A, A, dict(PIPE, host_pipeline_chunks=chunks))
+    assert st["decision"]["host_pipeline_chunks"] == chunks
+    assert st["decision"]["numeric_narrow_rows"] > 29000
+    check(A, A, C)
+
+
 def test_small_host_multiply_is_not_chunked():
     A = M.laplacian_2d(64, 64, seed=0)
     C, st = host_multiply(A, A, {})

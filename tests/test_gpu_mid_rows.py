@@ -153,20 +153,54 @@ def test_narrow_rows_run_a_warp_each(width, per_row, length):
     # spans at the limits of the numeric (1088) and symbolic (4096) narrow kernels,
     # A rows around one warp's entries, products around the 128 of the register
     # classes, B rows around the 8 entries that the narrow kernels ask for
-    # (1024 rows in the list: the fewest that the symbolic one looks through)
-    A, B = _narrow(1024, width, per_row, width + per_row, length=length)
+    # (4096 equal rows: enough for a warp each)
+    A, B = _narrow(4096, width, per_row, width + per_row, length=length)
+    narrow = per_row * min(length, width) > 128 and length >= 8
     for a, b in ((A, B), (A.widened(), B.widened())):
-        C, _ = multiply_device(a, b)
+        C, st = multiply_device(a, b)
         check(a, b, C)
+        assert st["decision"]["numeric_narrow_rows"] == (A.rows if narrow and width <= 1088 else 0)
+        assert st["decision"]["symbolic_narrow_rows"] == (A.rows if narrow and width <= 4096 else 0)
+
+
+def _rows_of(counts, b_rows, width, length, seed):
+    """A whose row r references counts[r] of the b_rows rows of B, each `length` columns of `width`."""
+    rng = np.random.default_rng(seed)
+    B = M.from_coo(b_rows, width, np.repeat(np.arange(b_rows), length), rng.integers(0, width, b_rows * length),
+                   rng.uniform(-1, 1, b_rows * length))
+    cols = np.concatenate([np.sort(rng.choice(b_rows, k, replace=False)) for k in counts])
+    return M.from_coo(len(counts), b_rows, np.repeat(np.arange(len(counts)), counts), cols,
+                      rng.uniform(-1, 1, cols.size)), B
+
+
+@pytest.mark.parametrize("wf", [0, 1])
+@pytest.mark.parametrize("rows,entries,light", [(3, 40000, 0), (300, 500, 0), (5, 20000, 6000), (0, 0, 6000)])
+def test_heavy_or_few_narrow_rows_stay_in_blocks(wf, rows, entries, light):
+    # rows with more products than a warp's share of the class, and classes with
+    # too few rows for a warp each, run in their block class
+    A, B = _rows_of([entries] * rows + [24] * light, 40000, 1000, 16, rows + 7)
+    C, st = multiply_device(A, B, {"force_workflow": wf})
+    check(A, B, C)
+    assert st["decision"]["workflow"] == wf
+    assert st["decision"]["numeric_narrow_rows"] == light
+    assert st["decision"]["symbolic_narrow_rows"] == (light if wf == 0 else 0)
+
+
+def test_small_skewed_product_has_no_narrow_rows():
+    A = M.rmat(10, 8, seed=1)
+    C, st = multiply_device(A, A)
+    check(A, A, C)
+    assert st["decision"]["numeric_narrow_rows"] == 0
 
 
 @pytest.mark.parametrize("wf", [0, 1])
 def test_narrow_rows_with_repeated_columns(wf):
     # B rows that hold a column twice: two lanes of one step meet
-    A, B = _narrow(1100, 700, 40, 9, repeat=True)
+    A, B = _narrow(2200, 700, 40, 9, repeat=True)
     C, st = multiply_device(A, B, {"force_workflow": wf})
     check(A, B, C)
     assert st["decision"]["workflow"] == wf
+    assert st["decision"]["numeric_narrow_rows"] == A.rows
 
 
 @pytest.mark.parametrize("scale", [0.3, 1.0])
