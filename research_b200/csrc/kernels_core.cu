@@ -152,7 +152,7 @@ __device__ __forceinline__ bool narrow_row(uint64_t p, uint64_t anz, uint64_t sp
 // otherwise the rows of more than 1.5 times the mean allowed are, so that nearly
 // equal rows are not split over two launches. Whole multiplies, one B200, every
 // narrow row a warp -> by this rule: power-law 2^10 rows of 16 entries 342 -> 239
-// us; 3 rows of 320000 products 3.93 -> 0.88 ms; 600 rows of 16000 products, B
+// us; 3 rows of 320000 products 3.93 -> 0.74 ms; 600 rows of 16000 products, B
 // rows of 16 entries, 1068 -> 899 us (1500 such rows stay narrow: 1078 us); 1000
 // rows of a 64-entry band 197 -> 181 us (1400 stay narrow: 197 us).
 static uint32_t narrow_limit(uint64_t rows, uint64_t products, uint64_t anz, int num_sms) {
@@ -1153,7 +1153,11 @@ __device__ __forceinline__ void block_run_chunk(const Csr<RP>& B, EnumSmem<NT>& 
 // products, and -1 otherwise. Long B rows (over 128 entries) stay with the
 // balanced enumeration, whose fast path walks them without a search and keeps
 // every warp busy on rows of one or two entries (power-law, symbolic hash_s:
-// 0.029 ms against 0.045 ms by groups).
+// 0.029 ms against 0.045 ms by groups). Rows of more than 2 NT A entries stay
+// there too (asked for by the callers): they fill its chunks, and by groups they
+// are a long chain of dependent loads (300 rows of 8000 entries, 1000 columns:
+// whole multiply 1131 us against 1274 us by groups; 600 rows 1471 against 1789 us;
+// 300 rows of 200 entries 814 us either way).
 template <int NT>
 __device__ __forceinline__ int group_lanes(uint64_t anz, uint32_t np, uint32_t maxb) {
   if (maxb > 128) return -1;
@@ -1527,7 +1531,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 16 : NT == 256 ? 5 : 1) k_sym_
           if (!(S.keys[d >> 5] & m)) atomicOr(&S.keys[d >> 5], m);
         }
       };
-      if (lg >= 0) {
+      if (lg >= 0 && a1 - a0 <= (uint64_t)(2 * NT)) {
         __syncthreads();
         group_for_each_product<NT, false>(A, B, a0, a1, lg, [&](uint32_t c, double) { mark(c); });
         __syncthreads();
@@ -1677,7 +1681,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B
           if (!(S.d.bits[d >> 5] & m)) atomicOr(&S.d.bits[d >> 5], m);
         }
       };
-      if (lg >= 0) {
+      if (lg >= 0 && a1 - a0 <= (uint64_t)(2 * NT)) {
         __syncthreads();
         group_for_each_product<NT, true>(A, B, a0, a1, lg, add);
         __syncthreads();

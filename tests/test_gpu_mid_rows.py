@@ -125,6 +125,16 @@ def test_uneven_b_rows_take_the_balanced_enumeration():
             _run(A, B, num, sym if sym != "hash_s" else "hash_m")
 
 
+@pytest.mark.parametrize("num", list(CLASSES))
+@pytest.mark.parametrize("edge", [-1, 0, 1])
+def test_rows_of_many_short_entries(num, edge):
+    # A rows at the 2 threads' worth of entries up to which lane groups walk them,
+    # dense numeric and marked symbolic form
+    threads, cap = CLASSES[num]
+    A, B = _rows_of([2 * threads + edge] * 3, 2 * threads + 1, cap // 2, 4, edge + 5)
+    _run(A, B, num, num)
+
+
 def _narrow(rows, width, per_row, seed, repeat=False, length=40):
     """Product whose rows span exactly `width` columns: every A row references
     `per_row` B rows of `length` columns inside the width."""
