@@ -229,6 +229,9 @@ void set_num_narrow(DevWork& w, const DevCounters* c, int num_sms, int chunks = 
 // Most window items of `rows` bitmap-class rows with `nnz` output entries, and
 // the bytes of one.
 uint64_t item_capacity(uint64_t rows, uint64_t nnz);
+// Whether window items are launched for `rows` rows with a saved bitmap and at
+// most `most` output entries.
+bool items_pay(uint64_t rows, uint64_t most, int num_sms);
 size_t item_bytes();
 
 // Words of DevWork::win_scratch for a device with num_sms SMs (one 2^20-bit

@@ -3695,6 +3695,16 @@ bool ensure_kernel_attributes(int dev) {
 
 uint64_t item_capacity(uint64_t rows, uint64_t nnz) { return nnz / (kItemV - 2048) + 3 * rows + 1; }
 size_t item_bytes() { return sizeof(WinItem); }
+// Rows of one item each are not spread over blocks, and the class's other rows
+// wait for the items' launch to end: with fewer than four such rows per SM that
+// idle time is more than the items save (numeric bitmap class of power-law 2^13
+// rows, whole -> items first: 6 entries a row, 11 items beside 1369 other rows,
+// 137 -> 194 us; 11 entries, 92 items, 233 -> 305 us; 16 entries, 296 items, 293
+// -> 326 us; 2^14 rows of 6 entries, 1917 items, 369 -> 315 us; of long rows few
+// are enough: 98 rows in 884 items, 3.6 -> 0.9 ms).
+bool items_pay(uint64_t rows, uint64_t most, int num_sms) {
+  return rows >= 4ull * num_sms || most > (uint64_t)kItemV;
+}
 
 void set_sym_narrow(DevWork& w, const DevCounters* c, int num_sms) {
   for (int k = 0; k < SB_COUNT; ++k) {

@@ -651,10 +651,13 @@ void prepare_windows(ocean_handle* h, uint64_t a_nnz, unsigned bitmap_rows) {
 }
 
 // Buffers of the window items for the numeric bitmap class's saved rows. If
-// they cannot be allocated, the rows run whole in k_num_bitmap (no error).
-void prepare_items(ocean_handle* h, unsigned bitmap_rows, uint64_t bitmap_nnz) {
+// they cannot be allocated, or the items are not worth launching, the rows run
+// whole in k_num_bitmap (no error).
+void prepare_items(ocean_handle* h, unsigned bitmap_rows, uint64_t bitmap_nnz, uint64_t b_cols) {
   h->w.items = nullptr;
   if (!h->w.bm_cache || bitmap_rows == 0 || h->cfg.numeric_windows) return;
+  if (!items_pay(h->h_ctr->sym_count[SB_BITMAP], std::min<uint64_t>(h->h_ctr->max_products, b_cols), h->num_sms))
+    return;
   const uint64_t cap = item_capacity(bitmap_rows, bitmap_nnz);
   if (cap > 0xFFFFFFFFull) return;
   auto try_grow = [](auto*& p, uint64_t& have, uint64_t need) {
@@ -1189,7 +1192,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         unsigned num_counts[NB_COUNT];
         for (int i = 0; i < NB_COUNT; ++i) num_counts[i] = h->h_ctr->num_count[i];
         prepare_windows(h, A.nnz, num_counts[NB_BITMAP]);
-        prepare_items(h, num_counts[NB_BITMAP], h->h_ctr->num_nnz[NB_BITMAP]);
+        prepare_items(h, num_counts[NB_BITMAP], h->h_ctr->num_nnz[NB_BITMAP], B.cols);
         set_num_narrow(h->w, h->h_ctr, h->num_sms, h->w.chunks);
         const OutSpec exact{h->w.rowptr64, h->w.row_nnz, nullptr, nullptr, nullptr};
         if (h->w.chunks) {

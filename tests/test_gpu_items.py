@@ -65,6 +65,16 @@ def test_items_hold_at_most_their_slots():
     assert C.nnz > span
 
 
+@pytest.mark.parametrize("scale,per_row,items", [(13, 8, False), (14, 8, True)])
+def test_few_rows_of_one_item_run_whole(scale, per_row, items):
+    # a few dozen rows of at most 8192 entries with a saved bitmap: no items; thousands: items
+    A = M.rmat(scale, per_row, seed=2)
+    C, st = multiply_device(A, A)
+    check(A, A, C)
+    assert st["decision"]["bitmap_cache_used_bytes"] > 0
+    assert (st["decision"]["window_item_rows"] > 0) == items
+
+
 @pytest.mark.parametrize("chunks", [2, 5])
 def test_items_in_the_host_pipeline(chunks):
     A, B = heavy_mix(b_rows=6000, cols=1 << 18, seed=8)
