@@ -12,8 +12,8 @@ from research_b200.ocean import SpGEMM
 
 pytestmark = pytest.mark.gpu
 
-# small inputs take the chunked path only with the product threshold at 0, the
-# analysis read-back forced (it is skipped below 1 M entries of A) and the
+# small inputs take the chunked path only with the product threshold at 0, as
+# inputs large enough for a choice of the workflow (small_problem_nnz) and in the
 # precise workflow (the only one that pipelines)
 PIPE = {"host_pipeline_min_products": 0, "small_problem_nnz": 0, "force_workflow": 0}
 

@@ -8,7 +8,9 @@ within 1e-12 * sum |a*b| (at most 3000 FP64 terms per entry in another order:
 below 3000 * 2^-53 = 3.4e-13 of it)."""
 import numpy as np
 import pytest
+import torch
 
+from oracle import oracle as O
 from research_b200 import matrices as M
 from research_b200.ocean import SpGEMM
 
@@ -17,7 +19,7 @@ from test_gpu_windows import heavy_mix
 
 pytestmark = pytest.mark.gpu
 
-FORCE = {"force_sym_bin": SYM_BINS["bitmap"], "force_num_bin": NUM_BINS["bitmap"]}
+FORCE = {"force_sym_bin": SYM_BINS["bitmap"], "force_num_bin": NUM_BINS["bitmap"], "force_workflow": 0}
 
 
 @pytest.mark.parametrize("cols", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, 1 << 20])
@@ -39,17 +41,33 @@ def test_power_law_rows(cols, wide_pointers):
 @pytest.mark.parametrize("span", [64, 2048, 2049, 1 << 18, (1 << 19) + 1, 1 << 20])
 @pytest.mark.parametrize("entries", [1, 255, 256, 257, 1025])
 def test_item_edges(span, entries):
-    # one row of `entries` B rows of 9 columns, and single-entry rows beside it
+    # rows of `entries` B rows of 9 columns and single-entry rows beside them, in
+    # numbers that let their bitmaps be saved and items be launched: 1100 copies
+    # of the row up to 2049 columns, one and a row of 12000 products beyond
     rng = np.random.default_rng(span + entries)
     r = np.repeat(np.arange(entries), 9)
     c = rng.integers(0, span, r.size)
     c[0], c[-1] = 0, span - 1
-    B = M.from_coo(entries, span, r, c, rng.uniform(-1, 1, r.size))
-    k = np.arange(entries)
-    A = M.from_coo(3, entries, np.r_[np.zeros(entries, int), 1, 2], np.r_[k, 0, entries - 1],
-                   rng.uniform(-1, 1, entries + 2))
-    C, _ = multiply_device(A, B, FORCE)
+    whole, extra = (1100, 0) if span <= 2049 else (1, 20)
+    for i in range(extra):
+        r = np.r_[r, np.full(600, entries + i)]
+        c = np.r_[c, rng.choice(span, 600, replace=False)]
+    B = M.from_coo(entries + extra, span, r, c, rng.uniform(-1, 1, r.size))
+    parts = [np.arange(entries)] * whole + [[0], [entries - 1]] + [entries + np.arange(extra)] * bool(extra)
+    ar = np.repeat(np.arange(len(parts)), [len(k) for k in parts])
+    A = M.from_coo(len(parts), entries + extra, ar, np.concatenate(parts), rng.uniform(-1, 1, ar.size))
+    C, st = multiply_device(A, B, FORCE)
     check(A, B, C)
+    prod, lo, hi = O.row_stats(A, B)
+    prod, width = prod.astype(np.int64), hi.astype(np.int64) - lo.astype(np.int64) + 1
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    cut = (width <= 1 << 18) | (prod > prod.sum() // (4 * sms))
+    words = -(-width[cut] // 64)
+    d = st["decision"]
+    assert d["bitmap_cache_used_bytes"] > 0 and d["window_item_rows"] == cut.sum()
+    # an item holds at most 256 groups of 32 words, and (here) no row more than 10240 entries
+    most = O.symbolic(A, B).max()
+    assert d["window_items"] == (-(-words // 8192)).sum() if most <= 10240 else d["window_items"] > cut.sum()
 
 
 def test_items_hold_at_most_their_slots():

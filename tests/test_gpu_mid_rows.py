@@ -6,7 +6,9 @@ sum |a_ik * b_kj| (FP64 sums of at most 4096 terms in another order: below
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from research_b200 import matrices as M
+from research_b200.ocean import HostCSR
 
 from test_gpu_parity import NUM_BINS, SYM_BINS, check, multiply_device
 
@@ -232,3 +234,41 @@ def test_narrow_rows_in_a_batch():
             for m, c in zip(ms, plan.run()):
                 check(m, m, c.download())
         plan.close()
+
+
+def _special(A):
+    """A with infinities, NaN and huge values among every 97th of its entries."""
+    v = A.val.copy()
+    at = np.arange(3, v.size, 97)
+    v[at] = np.resize([np.inf, 1.0, np.nan, -np.inf, 1e300, 0.0, -1.0], at.size)
+    return HostCSR(A.rows, A.cols, A.rowptr, A.col, v)
+
+
+@pytest.mark.parametrize("form", ["narrow", "dense", "bucket", "rank", "wide", "items"])
+def test_infinities_and_nan_stay_in_their_entries(form):
+    # every accumulator is cleared whatever it holds, so the rows that a block or
+    # a warp takes later are untouched
+    if form == "narrow":
+        A, cfg = M.banded(12000, 90, 20, seed=1), {}
+    elif form == "items":
+        A, cfg = M.rmat(14, 8, seed=2), {}
+    else:
+        cols = {"dense": 3000, "bucket": 60000, "rank": 60000, "wide": 3 << 20}[form]
+        k = {"dense": 30, "bucket": 30, "rank": 60, "wide": 30}[form]
+        A, B = _rows_of([k] * 4000, 3000, cols, 30, 3)
+        cfg = {"force_sym_bin": SYM_BINS["bitmap"], "force_num_bin": NUM_BINS["hash_m"]}
+    B = A if form in ("narrow", "items") else B
+    A = _special(A)
+    C, st = multiply_device(A, B, cfg)
+    if form == "narrow":
+        assert st["decision"]["numeric_narrow_rows"] > 11000
+    if form == "items":
+        assert st["decision"]["window_item_rows"] > 1000
+    with np.errstate(all="ignore"):
+        cp, cj, cx, ca = O.spgemm(A, B, with_abs=True)
+        assert np.array_equal(C.rowptr.astype(np.uint64), cp) and np.array_equal(C.col, cj)
+        nan, inf = np.isnan(cx), np.isinf(cx)
+        assert nan.any() and inf.any()
+        assert np.array_equal(np.isnan(C.val), nan) and np.array_equal(C.val[inf], cx[inf])
+        fine = ~(nan | inf)
+        assert (np.abs(C.val[fine] - cx[fine]) <= 1e-12 * ca[fine]).all()

@@ -71,9 +71,9 @@ def test_forced_classes_uniform(sym, num):
     check(A, A, C)
 
 
-@pytest.mark.parametrize("readback", [False, True])
+@pytest.mark.parametrize("choose", [False, True])
 @pytest.mark.parametrize("gen", ["uniform", "banded", "block", "rmat14", "rect"])
-def test_families(gen, readback):
+def test_families(gen, choose):
     if gen == "uniform":
         A = M.uniform_random(20000, 16, seed=1); B = A
     elif gen == "banded":
@@ -84,9 +84,11 @@ def test_families(gen, readback):
         A = M.rmat(14, 16, seed=4); B = A
     else:
         A = M.rect_poisson(16384, 65536, 12.0, seed=5); B = M.transpose(A)
-    # readback: class sizes read back after the analysis (selective launches, bitmap cache);
-    # otherwise the small-input mode that launches every class without a read-back
-    C, st = multiply_device(A, B, {"small_problem_nnz": 0 if readback else 1 << 30})
+    # choose: the workflow is chosen from the analysis, as for large inputs;
+    # otherwise the precise one, as for inputs of at most small_problem_nnz entries
+    C, st = multiply_device(A, B, {"small_problem_nnz": 0 if choose else 1 << 30})
+    if not choose:
+        assert st["decision"]["workflow"] == 0
     check(A, B, C)
     assert sum(st["binning_2"]) == int(np.count_nonzero(np.diff(C.rowptr.astype(np.int64))))
 

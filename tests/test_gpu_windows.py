@@ -66,8 +66,8 @@ def test_windowed_rows_match_oracle(cache, bits):
     A, B = heavy_mix()
     if bits == 64:
         A, B = A.widened(), B.widened()
-    # small_problem_nnz 0: read the class sizes back after the analysis, which
-    # lets the symbolic pass save bitmaps (cache > 0) for the numeric pass
+    # (small_problem_nnz 0: the workflow is chosen as for large inputs); the
+    # symbolic pass saves bitmaps for the numeric pass where cache > 0
     C, st = run(A, B, {"bitmap_cache_fraction": cache, "small_problem_nnz": 0, "numeric_windows": True})
     check(A, B, C)
     assert st["decision"]["numeric_bitmap_kernel"] == "window"

@@ -51,6 +51,18 @@ def test_noalloc_matches_regular_entry_point_twice(bits):
         assert np.array_equal(got, O.symbolic(A, A).astype(np.uint32))
 
 
+@pytest.mark.parametrize("gen", ["uniform", "banded", "block", "rmat", "rect", "laplacian"])
+def test_noalloc_launches_every_class(gen):
+    # without the class sizes on the host every class kernel runs at full grid,
+    # most of them here on an empty list
+    A = {"uniform": lambda: M.uniform_random(20000, 16, seed=1), "banded": lambda: M.banded(30000, 65, 24, seed=2),
+         "block": lambda: M.block_diagonal(32768, 256, 32, seed=3), "rmat": lambda: M.rmat(14, 16, seed=4),
+         "rect": lambda: M.rect_poisson(16384, 65536, 12.0, seed=5), "laplacian": lambda: M.laplacian_2d(64, 64)}[gen]()
+    B = M.transpose(A) if gen == "rect" else A
+    got = noalloc_counts(DeviceCSR.from_host(A), DeviceCSR.from_host(B))
+    assert np.array_equal(got, O.symbolic(A, B).astype(np.uint32))
+
+
 def test_noalloc_call_allocates_nothing():
     import torch
     A = M.rmat(16, 16, seed=34)
