@@ -68,10 +68,18 @@ struct DevWork {
   // most lane slots of a narrow row of each class (0: the narrow-row kernel is
   // not launched and every row runs in its class kernel)
   uint32_t sym_narrow[SB_COUNT] = {0}, num_narrow[NB_COUNT] = {0};
+  // kernel of each numeric hash class (HashForm): by the spans of its rows
+  uint8_t hash_form[NB_COUNT] = {0};
   // segment-driven dispatch: per-row policy slot (0: the call's policy,
   // 1 + SegClass: that segment class's policy); null: slot 0 for every row
   const uint8_t* row_pol = nullptr;
 };
+
+// Kernels of a numeric hash class: rows of up to 2^20 columns run in k_num_rank
+// and wider ones in k_num_hash (HF_BOTH; k_num_hash only where B has more than
+// 2^20 columns), or k_num_rank runs alone (no row is wider), or every row runs
+// in k_num_hash, which takes rows of any span (nearly all are wider).
+enum HashForm : uint8_t { HF_BOTH = 0, HF_RANK = 1, HF_HASH = 2 };
 
 constexpr int kScanTile = 1024;  // rows per scan tile: 1024 threads of k_scan_reduce, 256 x 4 of k_scan_apply
 inline uint64_t scan_tiles(uint64_t n) { return (n + kScanTile - 1) / kScanTile; }
@@ -225,6 +233,11 @@ void set_sym_narrow(DevWork& w, const DevCounters* c, int num_sms);
 // the scan made; null: not known, no narrow rows. chunks: row chunks of equal
 // products that the numeric phase runs in (0: none).
 void set_num_narrow(DevWork& w, const DevCounters* c, int num_sms, int chunks = 0);
+
+// DevWork::hash_form from the counters of the scan that made the class lists;
+// lists_change: the lists may be made again (a batch plan's runs), so HF_RANK,
+// which leaves wider rows unwritten, is not used. Null: not known, HF_BOTH.
+void set_hash_forms(DevWork& w, const DevCounters* c, bool lists_change = false);
 
 // Most window items of `rows` bitmap-class rows with `nnz` output entries, and
 // the bytes of one.

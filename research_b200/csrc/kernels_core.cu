@@ -1954,22 +1954,24 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_num_rank(Csr<RP> A, Csr<RP> B
 // Rows of the hash classes whose span exceeds 2^20 columns: open addressing in
 // shared memory, then a radix sort of packed (column offset, dense index)
 // words, or, when the span is too wide for the packing, a bitonic sort of
-// (column << 32 | slot) keys. Launched only for B of more than 2^20 columns;
-// the blocks stride over the class list and leave the other rows to
-// k_num_rank.
+// (column << 32 | slot) keys. Launched only where B has more than 2^20 columns.
+// all: every row of the list, taken one by one from the queue (2^21 uniform rows
+// of 16 entries, whole multiply: 37 ms, 42.5 ms when k_num_rank walked the list
+// first and the blocks strode over it); otherwise the blocks stride over the
+// list and leave the rows of up to 2^20 columns to k_num_rank.
 template <int NT, int LOG2T>
 struct NumHashSmem {
   double vals[1 << LOG2T];
   uint32_t keys[1 << LOG2T];  // reused as (1 << LOG2T) / 2 sort keys of 64 bits, or two radix buffers
   EnumSmem<NT> e;  // after the products: radix digit counts and dense-to-slot map
-  uint32_t s_n, s_acc;
+  uint32_t s_idx, s_n, s_acc;
 };
 
 template <typename RP, int NT, int LOG2T>
 __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue q, OutSpec o,
                                                  DevCounters* __restrict__ ctr, const uint32_t* __restrict__ lo,
                                                  const uint32_t* __restrict__ hi, uint32_t* __restrict__ c_col,
-                                                 double* __restrict__ c_val) {
+                                                 double* __restrict__ c_val, bool all) {
   constexpr int T = 1 << LOG2T;
   constexpr int PER = T / NT;
   constexpr int CAP = T / 2;  // sort capacity (entries) in the reused key area
@@ -1978,11 +1980,17 @@ __global__ void __launch_bounds__(NT) k_num_hash(Csr<RP> A, Csr<RP> B, RowQueue 
   NumHashSmem<NT, LOG2T>& S = *reinterpret_cast<NumHashSmem<NT, LOG2T>*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t count = *q.count;
-  for (uint32_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
+  for (uint32_t next = blockIdx.x;; next += gridDim.x) {
+    if (all) {
+      if (tid == 0) S.s_idx = atomicAdd(q.cursor, 1u);
+      __syncthreads();
+    }
+    const uint32_t idx = all ? S.s_idx : next;
+    if (idx >= count) break;
     const uint32_t row = q.rows[idx];
     const uint32_t rlo = lo[row];
     const uint32_t span1 = hi[row] - rlo;
-    if (span1 < (uint32_t)kBitmapBits) continue;
+    if (!all && span1 < (uint32_t)kBitmapBits) continue;
     const uint64_t a0 = A.row_begin(row), a1 = A.row_end(row);
     const uint32_t cap = o.cap[row];
     const uint64_t off = o.off[row];
@@ -3170,10 +3178,12 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
                                                      unsigned* __restrict__ chunk_count) {
   __shared__ unsigned long long scr[33];
   __shared__ unsigned long long s_cls[6][NB_COUNT];
+  __shared__ unsigned s_wide[NB_COUNT];
   __shared__ unsigned s_cnt[NB_COUNT * kMaxChunks];
   __shared__ uint32_t s_bound[kMaxChunks + 1];
   const int nseg = chunks > 1 ? chunks : 1;
   if (threadIdx.x < 6 * NB_COUNT) (&s_cls[0][0])[threadIdx.x] = 0ull;
+  if (threadIdx.x < NB_COUNT) s_wide[threadIdx.x] = 0u;
   if (threadIdx.x < NB_COUNT * kMaxChunks) s_cnt[threadIdx.x] = 0u;
   if (nseg > 1 && (int)threadIdx.x <= nseg) s_bound[threadIdx.x] = chunk_bound[threadIdx.x];
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * 4;
@@ -3203,9 +3213,10 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
   int bq[4], sq[4];
   uint32_t rq[4], aq[4], pq[4];
   bool nq[4];  // narrow rows, whatever their limit
+  bool wq[4];  // rows of the hash classes wider than 2^20 columns
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    nq[q] = false;
+    nq[q] = wq[q] = false;
     const uint64_t i = base + q;
     int b = -1;
     if (i < n) {
@@ -3221,6 +3232,7 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       if (b == NB_BITMAP && (uint64_t)hi[i] - lo[i] + 1 > kBitmapBits) atomicAdd(&ctr->num_wide, 1u);
       aq[q] = anz[i];
       pq[q] = p;
+      wq[q] = b >= NB_HASH_S && b <= NB_HASH_L && (uint64_t)hi[i] - lo[i] + 1 > kBitmapBits;
       nq[q] = (b == NB_HASH_S || b == NB_HASH_M) && pols.p[0].force_bin < 0 &&
               narrow_row(p, aq[q], (uint64_t)hi[i] - lo[i] + 1, kNarrowNum, 0xFFFFFFFFu);
     }
@@ -3263,7 +3275,11 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       atomicAdd(&s_cls[1][c], b2);
       atomicAdd(&s_cls[2][c], d);
     }
-    // the class's narrow rows
+    // the class's wide rows and its narrow rows
+    unsigned wide = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) wide += __popc(__ballot_sync(kFull, bq[q] == c && wq[q]));
+    if (lane == 0 && wide) atomicAdd(&s_wide[c], wide);
     bool any = false;
 #pragma unroll
     for (int q = 0; q < 4; ++q) any |= bq[q] == c && nq[q];
@@ -3292,6 +3308,7 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
     atomicAdd(&ctr->num_nnz[threadIdx.x], s_cls[0][threadIdx.x]);
     atomicAdd(&ctr->num_anz[threadIdx.x], s_cls[1][threadIdx.x]);
     atomicAdd(&ctr->num_prod[threadIdx.x], s_cls[2][threadIdx.x]);
+    if (s_wide[threadIdx.x]) atomicAdd(&ctr->hash_wide[threadIdx.x], s_wide[threadIdx.x]);
     if (s_cls[3][threadIdx.x]) {
       atomicAdd(&ctr->narrow_rows[threadIdx.x], s_cls[3][threadIdx.x]);
       atomicAdd(&ctr->narrow_anz[threadIdx.x], s_cls[4][threadIdx.x]);
@@ -3625,7 +3642,8 @@ constexpr size_t sym_hash_smem() { return sizeof(SymHashSmem<NT, LOG2T>); }
 
 int g_occ[24];  // resident blocks per SM of each persistent kernel (same order as kinds)
 enum Kind { K_SYM_ESC1, K_SYM_ESC2, K_SYM_ESC4, K_SYM_S, K_SYM_M, K_SYM_L, K_SYM_BM,
-            K_NUM_ESC1, K_NUM_ESC2, K_NUM_ESC4, K_NUM_S, K_NUM_M, K_NUM_L, K_NUM_BM, K_NUM_WIN };
+            K_NUM_ESC1, K_NUM_ESC2, K_NUM_ESC4, K_NUM_S, K_NUM_M, K_NUM_L, K_NUM_HASH_S, K_NUM_HASH_M,
+            K_NUM_HASH_L, K_NUM_BM, K_NUM_WIN };
 
 template <typename F>
 int occ_of(F f, int threads, size_t smem) {
@@ -3671,6 +3689,9 @@ void configure_kernel_attributes() {
   g_occ[K_NUM_ESC1] = occ_of(k_num_esc<uint32_t, 1>, 256, 0);
   g_occ[K_NUM_ESC2] = occ_of(k_num_esc<uint32_t, 2>, 256, 0);
   g_occ[K_NUM_ESC4] = occ_of(k_num_esc<uint32_t, 4>, 256, 0);
+  g_occ[K_NUM_HASH_S] = occ_of(k_num_hash<uint32_t, 128, 10>, 128, num_hash_smem<128, 10>());
+  g_occ[K_NUM_HASH_M] = occ_of(k_num_hash<uint32_t, 256, 12>, 256, num_hash_smem<256, 12>());
+  g_occ[K_NUM_HASH_L] = occ_of(k_num_hash<uint32_t, 512, 13>, 512, num_hash_smem<512, 13>());
   g_occ[K_NUM_S] = occ_of(k_num_rank<uint32_t, 128, 512>, 128, num_rank_smem<128, 512>());
   g_occ[K_NUM_M] = occ_of(k_num_rank<uint32_t, 256, 2048>, 256, num_rank_smem<256, 2048>());
   g_occ[K_NUM_L] = occ_of(k_num_rank<uint32_t, 512, 4096>, 512, num_rank_smem<512, 4096>());
@@ -3712,6 +3733,17 @@ void set_sym_narrow(DevWork& w, const DevCounters* c, int num_sms) {
     w.sym_narrow[k] = hash && c->sym_count[k] >= 1024 && c->sym_prod[k] >= 8 * c->sym_anz[k]
                           ? narrow_limit(c->sym_count[k], c->sym_prod[k], c->sym_anz[k], num_sms)
                           : 0u;
+  }
+}
+
+void set_hash_forms(DevWork& w, const DevCounters* c, bool lists_change) {
+  for (int k = 0; k < NB_COUNT; ++k) {
+    w.hash_form[k] = HF_BOTH;
+    if (!c) continue;
+    // a row passed over by k_num_rank costs it 2.6 ns (2^21 rows of 256 products);
+    // a row of up to 2^20 columns costs about 8 ns more in k_num_hash
+    if (4ull * c->hash_wide[k] > 3ull * c->num_count[k]) w.hash_form[k] = HF_HASH;
+    else if (c->hash_wide[k] == 0 && !lists_change) w.hash_form[k] = HF_RANK;
   }
 }
 
@@ -3900,7 +3932,9 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
     return RowQueue{w.num_bins + (uint64_t)c * A.rows, w.ctr->num_count + c, w.ctr->num_cursor + c};
   };
   unsigned gsz;
-  const bool wide = B.cols > kBitmapBits;  // only then can a row's span exceed 2^20 columns
+  auto rank = [&](int cls) { return w.hash_form[cls] != HF_HASH; };
+  // (only where B has more than 2^20 columns can a row's span exceed them)
+  auto hash = [&](int cls) { return w.hash_form[cls] != HF_RANK && B.cols > kBitmapBits; };
   mark(NB_ESC1);
   if ((gsz = grid(K_NUM_ESC1, NB_ESC1, 8)) && ++launched)
     k_num_esc<RP, 1><<<gsz, 256, 0, s>>>(A, B, queue(NB_ESC1), o, w.ctr, c_col, c_val);
@@ -3920,31 +3954,31 @@ int launch_numeric(const Csr<RP>& A, const Csr<RP>& B, const DevWork& w, const O
                                                        w.num_narrow[cls], w.ctr->num_narrow_done + cls);
   };
   mark(NB_HASH_S);
-  narrow(NB_HASH_S);
-  if ((gsz = grid(K_NUM_S, NB_HASH_S, 1)) && ++launched)
+  if (rank(NB_HASH_S)) narrow(NB_HASH_S);
+  if (rank(NB_HASH_S) && (gsz = grid(K_NUM_S, NB_HASH_S, 1)) && ++launched)
     k_num_rank<RP, 128, 512><<<gsz, 128, num_rank_smem<128, 512>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.prod, w.maxb,
                                                                   w.lo, w.hi, c_col, c_val,
                                                                   narrow_done(NB_HASH_S));
-  if (wide && gsz && ++launched)
+  if (hash(NB_HASH_S) && (gsz = grid(K_NUM_HASH_S, NB_HASH_S, 1)) && ++launched)
     k_num_hash<RP, 128, 10><<<gsz, 128, num_hash_smem<128, 10>(), s>>>(A, B, queue(NB_HASH_S), o, w.ctr, w.lo, w.hi,
-                                                                  c_col, c_val);
+                                                                  c_col, c_val, !rank(NB_HASH_S));
   mark(NB_HASH_M);
-  narrow(NB_HASH_M);
-  if ((gsz = grid(K_NUM_M, NB_HASH_M, 1)) && ++launched)
+  if (rank(NB_HASH_M)) narrow(NB_HASH_M);
+  if (rank(NB_HASH_M) && (gsz = grid(K_NUM_M, NB_HASH_M, 1)) && ++launched)
     k_num_rank<RP, 256, 2048><<<gsz, 256, num_rank_smem<256, 2048>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.prod, w.maxb,
                                                                   w.lo, w.hi, c_col, c_val,
                                                                   narrow_done(NB_HASH_M));
-  if (wide && gsz && ++launched)
+  if (hash(NB_HASH_M) && (gsz = grid(K_NUM_HASH_M, NB_HASH_M, 1)) && ++launched)
     k_num_hash<RP, 256, 12><<<gsz, 256, num_hash_smem<256, 12>(), s>>>(A, B, queue(NB_HASH_M), o, w.ctr, w.lo, w.hi,
-                                                                  c_col, c_val);
+                                                                  c_col, c_val, !rank(NB_HASH_M));
   mark(NB_HASH_L);
-  if ((gsz = grid(K_NUM_L, NB_HASH_L, 1)) && ++launched)
+  if (rank(NB_HASH_L) && (gsz = grid(K_NUM_L, NB_HASH_L, 1)) && ++launched)
     k_num_rank<RP, 512, 4096><<<gsz, 512, num_rank_smem<512, 4096>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.prod, w.maxb,
                                                                   w.lo, w.hi, c_col, c_val,
                                                                   NarrowDone{0u, nullptr});
-  if (wide && gsz && ++launched)
+  if (hash(NB_HASH_L) && (gsz = grid(K_NUM_HASH_L, NB_HASH_L, 1)) && ++launched)
     k_num_hash<RP, 512, 13><<<gsz, 512, num_hash_smem<512, 13>(), s>>>(A, B, queue(NB_HASH_L), o, w.ctr, w.lo, w.hi,
-                                                                  c_col, c_val);
+                                                                  c_col, c_val, !rank(NB_HASH_L));
   mark(NB_BITMAP);
   const bool windowed = !o.count && w.win_cursor && w.win_scratch;
   if (windowed) {

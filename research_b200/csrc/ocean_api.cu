@@ -1152,6 +1152,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         const OutSpec est_out{h->w.est_off, h->w.est, h->w.cnt, h->w.ovf, &h->w.ctr->overflow_n};
         st.bm_kernel = num_counts[NB_BITMAP] ? 1 : 0;
         set_num_narrow(h->w, class_counts ? h->h_ctr : nullptr, h->num_sms);
+        set_hash_forms(h->w, class_counts ? h->h_ctr : nullptr);
         st.launches += launch_numeric(A, B, h->w, est_out, (uint32_t*)t_col, (double*)t_val, h->num_sms, s,
                                       track ? h->ev + EV_NUM0 : nullptr, class_counts ? num_counts : nullptr);
         if (track) h->ev_mask |= ((1ull << (NB_COUNT + 1)) - 1) << EV_NUM0;
@@ -1194,6 +1195,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         prepare_windows(h, A.nnz, num_counts[NB_BITMAP]);
         prepare_items(h, num_counts[NB_BITMAP], h->h_ctr->num_nnz[NB_BITMAP], B.cols);
         set_num_narrow(h->w, h->h_ctr, h->num_sms, h->w.chunks);
+        set_hash_forms(h->w, h->h_ctr);
         const OutSpec exact{h->w.rowptr64, h->w.row_nnz, nullptr, nullptr, nullptr};
         if (h->w.chunks) {
           st.launches += pipeline_numeric(h, A, B, exact, owner, nnz, bits, s);
@@ -1630,6 +1632,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
       b->c_nnz = b->h_ctr->total_nnz;
       for (int i = 0; i < NB_COUNT; ++i) b->num_counts[i] = b->h_ctr->num_count[i];
       set_num_narrow(w, b->h_ctr, h->num_sms);
+      set_hash_forms(w, b->h_ctr, true);
     } else {
       launch_batch_guard(w.ctr, &w.ctr->total_nnz, b->c_nnz, s);
       launched += 1;
@@ -1656,6 +1659,7 @@ void batch_pipeline(ocean_batch* b, cudaStream_t s, bool plan) {
       b->total_est = b->h_ctr->total_est;
       for (int i = 0; i < NB_COUNT; ++i) b->num_counts[i] = b->h_ctr->num_count[i];
       set_num_narrow(w, b->h_ctr, h->num_sms);
+      set_hash_forms(w, b->h_ctr, true);
       OCEAN_CUDA(cudaMalloc((void**)&b->t_col, std::max<uint64_t>(b->total_est, 1) * 4));
       OCEAN_CUDA(cudaMalloc((void**)&b->t_val, std::max<uint64_t>(b->total_est, 1) * 8));
     } else {

@@ -236,6 +236,27 @@ def test_narrow_rows_in_a_batch():
         plan.close()
 
 
+@pytest.mark.parametrize("wf", [0, 1, 2])
+@pytest.mark.parametrize("narrow_part", [0.0, 0.2, 0.3, 0.97, 1.0])
+def test_rows_wider_than_a_bitmap_among_others(wf, narrow_part):
+    # classes whose rows are all, mostly, partly or never wider than 2^20 columns:
+    # the hash kernel takes the class whole from three quarters wide rows on
+    rng = np.random.default_rng(int(100 * narrow_part) + wf)
+    b_rows, cols, n = 6000, 3 << 20, 2000
+    top = np.where(np.arange(b_rows) < b_rows // 2, 1 << 19, cols)  # the first half stays below 2^19 columns
+    r = np.repeat(np.arange(b_rows), 16)
+    B = M.from_coo(b_rows, cols, r, (rng.random(r.size) * top[r]).astype(np.int64), rng.uniform(-1, 1, r.size))
+    k = rng.choice([12, 60, 200], n)  # one class each
+    half = b_rows // 2
+    ac = np.concatenate([np.sort(rng.choice(half, m, replace=False)) + (0 if i < narrow_part * n else half)
+                         for i, m in enumerate(k)])
+    A = M.from_coo(n, b_rows, np.repeat(np.arange(n), k), ac, rng.uniform(-1, 1, ac.size))
+    for a, b in ((A, B), (A.widened(), B.widened())):
+        C, st = multiply_device(a, b, {"force_workflow": wf})
+        check(a, b, C)
+        assert all(st["binning_2"][NUM_BINS[c]] for c in CLASSES)
+
+
 def _special(A):
     """A with infinities, NaN and huge values among every 97th of its entries."""
     v = A.val.copy()
