@@ -1163,7 +1163,7 @@ __device__ __forceinline__ int group_lanes(uint64_t anz, uint32_t np, uint32_t m
   if (maxb > 128) return -1;
   const int lg = maxb <= 4 ? 2 : min(5, 32 - __clz(maxb - 1));
   const uint64_t pad = ((uint64_t)maxb + (1u << lg) - 1) >> lg << lg;
-  const uint64_t entries = (anz + (NT >> lg) - 1) / (NT >> lg) * (NT >> lg);
+  const uint64_t entries = (anz + (NT >> lg) - 1) & ~(uint64_t)((NT >> lg) - 1);
   return entries * pad <= 3ull * np ? lg : -1;
 }
 
@@ -1518,10 +1518,10 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 16 : NT == 256 ? 5 : 1) k_sym_
       __syncthreads();
       continue;
     }
-    const int lg = group_lanes<NT>(a1 - a0, np, maxb[row]);
     unsigned cnt = 0;
     const uint32_t nw = (span1 >> 5) + 1;
     if (nw <= T && nw <= np) {
+      const int lg = group_lanes<NT>(a1 - a0, np, maxb[row]);
 #pragma unroll 1
       for (uint32_t i = tid; i < nw; i += NT) S.keys[i] = 0u;
       auto mark = [&](uint32_t c) {
