@@ -524,6 +524,13 @@ void make_segment_policies(const Config& c, const SymPolicy& sp, const NumPolicy
 const SymPolicy* seg_sym(const ocean_handle* h) { return h->seg_dispatch ? h->seg_sp : nullptr; }
 const NumPolicy* seg_num(const ocean_handle* h) { return h->seg_dispatch ? h->seg_np : nullptr; }
 
+// Zeroes the counts, cursors and sums of the numeric classes, for a second scan
+// that makes their lists in the same call.
+void clear_numeric_classes(DevCounters* ctr, cudaStream_t s) {
+  constexpr size_t a = offsetof(DevCounters, num_count), b = offsetof(DevCounters, num_wide) + sizeof(unsigned);
+  OCEAN_CUDA(cudaMemsetAsync(reinterpret_cast<unsigned char*>(ctr) + a, 0, b - a, s));
+}
+
 // Phase 1: row analysis. The counters (class sizes, product totals) are read
 // back, so that only the classes that have rows are launched: for a small
 // input one read-back (about 10 us) costs less than the launches of five
@@ -1104,7 +1111,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
         st.total_est = h->h_ctr->total_est;
         if (!fits_device(h, 12.0 * (double)st.total_est, 0.45)) {
           wf = WF_PRECISE;  // the temporary output would not fit: count exactly instead
-          OCEAN_CUDA(cudaMemsetAsync(h->w.ctr->num_count, 0, sizeof(unsigned) * NB_COUNT * 2, s));
+          clear_numeric_classes(h->w.ctr, s);
         }
       }
       // host-buffer multiplies of many products: the numeric phase runs in

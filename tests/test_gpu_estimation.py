@@ -6,7 +6,7 @@ import pytest
 
 from oracle import oracle as O
 from research_b200 import matrices as M
-from research_b200.ocean import DeviceCSR, SpGEMM
+from research_b200.ocean import DeviceCSR, HostCSR, SpGEMM
 
 pytestmark = pytest.mark.gpu
 
@@ -107,3 +107,29 @@ def test_stats_queries_leave_no_cuda_error():
     x = torch.ones(1000, device="cuda") * 2  # would raise if an error were pending
     torch.cuda.synchronize()
     assert float(x.sum()) == 2000.0
+
+
+def test_precise_after_an_estimate_that_does_not_fit():
+    # 8.6 G product slots (103 GB) for 34 M entries: the estimated workflow gives
+    # way to exact counting, and the class sums are those of the exact lists alone
+    n, b = 131072, 256
+    rng = np.random.default_rng(1)
+    col = (np.arange(n)[:, None] // b * b + np.arange(b)[None, :]).astype(np.uint32).ravel()
+    A = HostCSR(n, n, (np.arange(n + 1) * b).astype(np.uint32), col, rng.uniform(-1, 1, col.size))
+    g = SpGEMM({"force_workflow": 2, "small_problem_nnz": 1 << 30})
+    dA = DeviceCSR.from_host(A)
+    C = g.multiply(dA, dA)
+    st = g.get_stats()
+    assert st["decision"]["workflow"] == 0 and C.nnz == n * b
+    numeric = st["classes"]["numeric"].values()
+    assert sum(c["nnz"] for c in numeric) == C.nnz
+    assert sum(c["products"] for c in numeric) == st["stats"]["intermediate_product"]
+    assert sum(c["a_nnz"] for c in numeric) == A.nnz
+    for r0 in (0, n // 2, n - b):
+        rp, cj, cx = C.download_rows(r0, r0 + b)
+        block = A.val[r0 * b:(r0 + b) * b].reshape(b, b)
+        assert np.array_equal(cj, A.col[r0 * b:(r0 + b) * b])
+        # 256 FP64 terms in another order: below 256 * 2^-53 = 2.8e-14 of sum |a*b|
+        assert (np.abs(cx.reshape(b, b) - block @ block) <= 1e-13 * (np.abs(block) @ np.abs(block))).all()
+    C.free()
+    g.close()
