@@ -187,7 +187,9 @@ struct Config {
   int force_sym_bin = -1;         // testing: put every non-empty row in one symbolic class
   int force_num_bin = -1;         // testing: put every non-empty row in one numeric class
   bool sync_on_return = true;     // check device status before returning
-  double bitmap_cache_fraction = 0.25;  // share of free device memory the saved row bitmaps may use
+  // share of device memory the saved row bitmaps may use: of 4% of the whole
+  // device without a look at what is free, beyond that of the free memory
+  double bitmap_cache_fraction = 0.25;
   int small_problem_nnz = 1 << 20;      // A with at most this many entries: precise workflow unless forced
   int spin_wait_us = 2000;              // poll the stream this long before a blocking synchronize
   int force_workflow = -1;              // -1 auto; 0 precise, 1 estimation (HLL), 2 ultra-sparse, 3 fat

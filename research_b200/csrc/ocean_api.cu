@@ -136,6 +136,24 @@ void grow(T*& p, uint64_t& cap, uint64_t need) {
   cap = n;
 }
 
+// The same with an eighth of headroom, for needs that follow the size of C
+// (every growth stalls the device); false if the memory cannot be had.
+template <typename T>
+bool try_grow(T*& p, uint64_t& cap, uint64_t need) {
+  if (p && cap >= need) return true;
+  if (p) cudaFree(p);
+  p = nullptr;
+  cap = 0;
+  const uint64_t n = need + need / 8;
+  if (cudaMalloc((void**)&p, n * sizeof(T)) != cudaSuccess) {
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
+  cap = n;
+  return true;
+}
+
 template <typename T>
 void grow_host(T*& p, uint64_t& cap, uint64_t need) {
   if (need <= cap && p) return;
@@ -637,21 +655,8 @@ void prepare_windows(ocean_handle* h, uint64_t a_nnz, unsigned bitmap_rows) {
   if (!h->cfg.numeric_windows || bitmap_rows == 0) return;
   const uint64_t need_cur = h->h_ctr->max_a_nnz > (unsigned)kBitmapThreads ? a_nnz : 1;
   const uint64_t need_scr = window_scratch_words(h->num_sms);
-  auto try_grow = [](auto*& p, uint64_t& cap, uint64_t need, size_t elem) {
-    if (p && cap >= need) return true;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    if (cudaMalloc((void**)&p, need * elem) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-      return false;
-    }
-    cap = need;
-    return true;
-  };
-  if (!try_grow(h->win_cursor, h->win_cursor_cap, need_cur, sizeof(uint32_t))) return;
-  if (!try_grow(h->win_scratch, h->win_scratch_cap, need_scr, sizeof(unsigned long long))) return;
+  if (!try_grow(h->win_cursor, h->win_cursor_cap, need_cur)) return;
+  if (!try_grow(h->win_scratch, h->win_scratch_cap, need_scr)) return;
   h->w.win_cursor = h->win_cursor;
   h->w.win_scratch = h->win_scratch;
   h->st.bm_kernel = 2;
@@ -667,19 +672,6 @@ void prepare_items(ocean_handle* h, unsigned bitmap_rows, uint64_t bitmap_nnz, u
     return;
   const uint64_t cap = item_capacity(bitmap_rows, bitmap_nnz);
   if (cap > 0xFFFFFFFFull) return;
-  auto try_grow = [](auto*& p, uint64_t& have, uint64_t need) {
-    if (p && have >= need) return true;
-    if (p) cudaFree(p);
-    p = nullptr;
-    have = 0;
-    if (cudaMalloc((void**)&p, need * sizeof(*p)) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-      return false;
-    }
-    have = need;
-    return true;
-  };
   uint64_t one = h->item_ctr ? 1 : 0;
   if (!try_grow(h->item_buf, h->item_buf_cap, cap * item_bytes()) ||
       !try_grow(h->item_rest, h->item_rest_cap, bitmap_rows) || !try_grow(h->item_ctr, one, 1))
@@ -693,7 +685,9 @@ void prepare_items(ocean_handle* h, unsigned bitmap_rows, uint64_t bitmap_nnz, u
 // Phase 2 of the precise workflow: symbolic class kernels (exact counts into
 // w.row_nnz) and, with_scan, the row-pointer scan and numeric class lists; the
 // counters are read back at the end. With allow_cache, bitmap-class rows save
-// their bitmaps into h->w.bm_cache, whose size comes from the analysis and is capped by bitmap_cache_fraction of free memory.
+// their bitmaps into h->w.bm_cache, whose size comes from the analysis and is
+// bounded by bitmap_cache_fraction of 4% of the device's memory, or, where that
+// is not enough, of the memory then free; a buffer that is there is used whole.
 template <typename RP>
 void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool with_scan,
                   bool allow_cache) {
@@ -707,15 +701,18 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
     // The free-memory query stalls the host for up to 10 ms when large results
     // were just freed (power-law 2^17, the previous C still pending: 28 ms per
     // multiply with it, 16 ms without): it is left out when the buffer of an
-    // earlier call is large enough, or when the bitmaps would fit their share
-    // of 4% of the device (an allocation that fails only turns the cache off).
+    // earlier call is large enough, or when the bitmaps fit their share of 4% of
+    // the whole device (an allocation that fails only turns the cache off).
+    // Buffers get an eighth of headroom within either bound: each growth frees
+    // and allocates, which waits for the device (24 products whose bitmaps grow
+    // by 2% each: 49.6 ms without headroom, 33 ms when nothing grows).
     const double share = h->cfg.bitmap_cache_fraction;
+    const uint64_t unasked = (uint64_t)(share * 0.04 * (double)h->device_bytes) / 8;
     uint64_t budget = 0;
     if (want >= 1024) {
-      if ((h->cache_buf && h->cache_cap_words >= want) || 8.0 * (double)want <= share * 0.04 * (double)h->device_bytes)
-        budget = want;
-      else
-        budget = (uint64_t)(share * (double)available_device_bytes(h->device)) / 8;
+      if (h->cache_buf && h->cache_cap_words >= want) budget = want;
+      else if (want <= unasked) budget = unasked;
+      else budget = (uint64_t)(share * (double)available_device_bytes(h->device)) / 8;
     }
     const uint64_t words = std::min(want, budget);
     if (words >= 1024) {
@@ -723,7 +720,7 @@ void run_symbolic(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStrea
         if (h->cache_buf) cudaFree(h->cache_buf);
         h->cache_buf = nullptr;
         h->cache_cap_words = 0;
-        const uint64_t grow_to = std::max(words, std::min(budget, words + words / 8));
+        const uint64_t grow_to = std::min(budget, words + words / 8);
         if (cudaMalloc((void**)&h->cache_buf, grow_to * 8) == cudaSuccess) {
           h->cache_cap_words = grow_to;
         } else {

@@ -12,7 +12,7 @@ import torch
 
 from oracle import oracle as O
 from research_b200 import matrices as M
-from research_b200.ocean import SpGEMM
+from research_b200.ocean import DeviceCSR, SpGEMM
 
 from test_gpu_parity import NUM_BINS, SYM_BINS, check, multiply_device
 from test_gpu_windows import heavy_mix
@@ -101,3 +101,26 @@ def test_items_in_the_host_pipeline(chunks):
     check(A, B, C)
     d = g.get_stats()["decision"]
     assert d["host_pipeline_chunks"] == chunks and d["window_item_rows"] > 0
+
+
+def test_growing_bitmaps_are_not_allocated_again_each_time():
+    # the second product's bitmaps take 5% more than the first's
+    rng = np.random.default_rng(4)
+    b_rows, cols, n, k = 2000, 1 << 18, 2000, 60
+    top = np.where(np.arange(b_rows) < b_rows // 2, 1 << 17, int(1.05 * (1 << 17)))
+    r = np.repeat(np.arange(b_rows), 300)
+    dB = DeviceCSR.from_host(M.from_coo(b_rows, cols, r, (rng.random(r.size) * top[r]).astype(np.int64),
+                                        rng.uniform(-1, 1, r.size)))
+    ac = np.concatenate([np.sort(rng.choice(b_rows // 2, k, replace=False)) for _ in range(n)])
+    first, second = (DeviceCSR.from_host(M.from_coo(n, b_rows, np.repeat(np.arange(n), k), ac + shift,
+                                                    rng.uniform(-1, 1, ac.size))) for shift in (0, b_rows // 2))
+    warm, g = SpGEMM(), SpGEMM()
+    warm.multiply(second, dB).free()  # the pool of C holds enough from here on
+    words, free = [], []
+    for A in (first, second):
+        g.multiply(A, dB).free()
+        torch.cuda.synchronize()
+        words.append(g.get_stats()["decision"]["bitmap_cache_bytes"])
+        free.append(torch.cuda.mem_get_info()[0])
+    assert 1.02 * words[0] < words[1] < 1.1 * words[0]
+    assert free[1] == free[0]
