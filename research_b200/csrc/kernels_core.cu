@@ -3212,11 +3212,11 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
   }
   int bq[4], sq[4];
   uint32_t rq[4], aq[4], pq[4];
-  bool nq[4];  // narrow rows, whatever their limit
-  bool wq[4];  // rows of the hash classes wider than 2^20 columns
+  // rows of the hash classes: narrow ones, whatever their limit (bit q), and
+  // those wider than 2^20 columns (bit 4 + q)
+  unsigned special = 0;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    nq[q] = wq[q] = false;
     const uint64_t i = base + q;
     int b = -1;
     if (i < n) {
@@ -3232,9 +3232,12 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       if (b == NB_BITMAP && (uint64_t)hi[i] - lo[i] + 1 > kBitmapBits) atomicAdd(&ctr->num_wide, 1u);
       aq[q] = anz[i];
       pq[q] = p;
-      wq[q] = b >= NB_HASH_S && b <= NB_HASH_L && (uint64_t)hi[i] - lo[i] + 1 > kBitmapBits;
-      nq[q] = (b == NB_HASH_S || b == NB_HASH_M) && pols.p[0].force_bin < 0 &&
-              narrow_row(p, aq[q], (uint64_t)hi[i] - lo[i] + 1, kNarrowNum, 0xFFFFFFFFu);
+      if (b >= NB_HASH_S && b <= NB_HASH_L) {
+        const uint64_t span = (uint64_t)hi[i] - lo[i] + 1;
+        if (span > kBitmapBits) special |= 16u << q;
+        else if (b != NB_HASH_L && pols.p[0].force_bin < 0 && narrow_row(p, aq[q], span, kNarrowNum, 0xFFFFFFFFu))
+          special |= 1u << q;
+      }
     }
     bq[q] = b;
     rq[q] = (uint32_t)i;
@@ -3275,31 +3278,32 @@ __global__ void __launch_bounds__(kScanApplyThreads) k_scan_apply(const uint32_t
       atomicAdd(&s_cls[1][c], b2);
       atomicAdd(&s_cls[2][c], d);
     }
-    // the class's wide rows and its narrow rows
-    unsigned wide = 0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) wide += __popc(__ballot_sync(kFull, bq[q] == c && wq[q]));
-    if (lane == 0 && wide) atomicAdd(&s_wide[c], wide);
-    bool any = false;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) any |= bq[q] == c && nq[q];
-    if (__any_sync(kFull, any)) {
-      unsigned long long r = 0, e = 0, f = 0;
+  }
+  if (__any_sync(kFull, special != 0)) {
+    for (int c = NB_HASH_S; c <= NB_HASH_L; ++c) {
+      unsigned wide = 0, rows = 0;
+      unsigned long long a = 0, d = 0;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        if (bq[q] == c && nq[q]) {
-          ++r;
-          e += aq[q];
-          f += pq[q];
+        if (bq[q] != c) continue;
+        wide += (special >> (4 + q)) & 1u;
+        if ((special >> q) & 1u) {
+          ++rows;
+          a += aq[q];
+          d += pq[q];
         }
       }
-      r = warp_sum_u64(r);
-      e = warp_sum_u64(e);
-      f = warp_sum_u64(f);
-      if (lane == 0) {
-        atomicAdd(&s_cls[3][c], r);
-        atomicAdd(&s_cls[4][c], e);
-        atomicAdd(&s_cls[5][c], f);
+      wide = __reduce_add_sync(kFull, wide);
+      rows = __reduce_add_sync(kFull, rows);
+      if (lane == 0 && wide) atomicAdd(&s_wide[c], wide);
+      if (rows) {
+        a = warp_sum_u64(a);
+        d = warp_sum_u64(d);
+        if (lane == 0) {
+          atomicAdd(&s_cls[3][c], (unsigned long long)rows);
+          atomicAdd(&s_cls[4][c], a);
+          atomicAdd(&s_cls[5][c], d);
+        }
       }
     }
   }

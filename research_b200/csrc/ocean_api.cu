@@ -545,8 +545,12 @@ const NumPolicy* seg_num(const ocean_handle* h) { return h->seg_dispatch ? h->se
 // Zeroes the counts, cursors and sums of the numeric classes, for a second scan
 // that makes their lists in the same call.
 void clear_numeric_classes(DevCounters* ctr, cudaStream_t s) {
-  constexpr size_t a = offsetof(DevCounters, num_count), b = offsetof(DevCounters, num_wide) + sizeof(unsigned);
-  OCEAN_CUDA(cudaMemsetAsync(reinterpret_cast<unsigned char*>(ctr) + a, 0, b - a, s));
+  auto zero = [&](size_t from, size_t to) {
+    OCEAN_CUDA(cudaMemsetAsync(reinterpret_cast<unsigned char*>(ctr) + from, 0, to - from, s));
+  };
+  zero(offsetof(DevCounters, num_count), offsetof(DevCounters, sym_anz));
+  zero(offsetof(DevCounters, num_wide), offsetof(DevCounters, usp_tile));
+  zero(offsetof(DevCounters, num_narrow_done), offsetof(DevCounters, item_rows));
 }
 
 // Phase 1: row analysis. The counters (class sizes, product totals) are read

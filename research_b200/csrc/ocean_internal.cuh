@@ -50,20 +50,11 @@ struct DevCounters {
   unsigned int max_a_nnz;
   unsigned int sym_count[SB_COUNT];
   unsigned int sym_cursor[SB_COUNT];
-  // the numeric classes, from num_count to num_wide: a scan that makes the class
-  // lists again starts from zeros (clear_numeric_classes)
   unsigned int num_count[NB_COUNT];
   unsigned int num_cursor[NB_COUNT];
   unsigned long long num_nnz[NB_COUNT];   // output entries per numeric class
   unsigned long long num_anz[NB_COUNT];   // A entries of the rows of each numeric class
   unsigned long long num_prod[NB_COUNT];  // products of the rows of each numeric class
-  unsigned long long narrow_rows[NB_COUNT];  // narrow rows of each numeric class, whatever their limit,
-  unsigned long long narrow_anz[NB_COUNT];   // their A entries
-  unsigned long long narrow_prod[NB_COUNT];  // and products
-  unsigned int num_narrow_done[NB_COUNT];  // rows of each class that k_num_narrow has written
-  unsigned int hash_wide[NB_COUNT];  // rows of each numeric hash class whose column span exceeds 2^20 columns
-  unsigned int wide_cursor;  // queue cursor of the kernel of the rows in num_wide (k_num_bitmap beside k_num_window)
-  unsigned int num_wide;     // numeric bitmap-class rows whose column span exceeds one 2^20-bit bitmap
   unsigned long long sym_anz[SB_COUNT];   // A entries of the rows of each symbolic class
   unsigned long long sym_prod[SB_COUNT];  // products of the rows of each symbolic class
   unsigned long long sym_words;           // bitmap words of single-window bitmap-class rows
@@ -77,11 +68,19 @@ struct DevCounters {
   double sample_compaction;               // HLL sampling: sum of products / estimate over samples
   unsigned int status;     // OR of DevError bits
   unsigned int err_row;
+  unsigned int num_wide;     // numeric bitmap-class rows whose column span exceeds one 2^20-bit bitmap
+  unsigned int wide_cursor;  // queue cursor of those rows' kernel (k_num_bitmap beside k_num_window)
   unsigned int usp_tile;     // fused ultra-sparse multiply: tiles handed out
   unsigned int num_long;     // rows of A listed as long (more than kLongRowEntries entries)
   unsigned int long_chunks;  // chunks of kLongChunk A entries of the listed rows
   unsigned int pad[1];
   unsigned int sym_narrow_done[SB_COUNT];  // rows of each class that k_sym_narrow has counted
+  unsigned int num_narrow_done[NB_COUNT];  // rows of each class that k_num_narrow has written
+  unsigned int hash_wide[NB_COUNT];  // rows of each numeric hash class whose column span exceeds 2^20 columns
+  unsigned int pad2[1];
+  unsigned long long narrow_rows[NB_COUNT];  // narrow rows of each numeric class, whatever their limit,
+  unsigned long long narrow_anz[NB_COUNT];   // their A entries
+  unsigned long long narrow_prod[NB_COUNT];  // and products
   unsigned int item_rows;    // numeric bitmap-class rows cut into window items
   unsigned int item_count;   // their window items
 };
