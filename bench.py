@@ -530,6 +530,8 @@ def run_ours(args, world, rank, local):
             traffic = json.loads(tfile.read_text()).get(dom)
         except Exception:
             traffic = None
+        if dom == "numeric_bitmap" and st["decision"].get("window_item_rows"):
+            traffic = None  # measured for k_num_bitmap alone, and window items ran in the class too
     comp = compulsory_bytes(A, B, nnz_c)
 
     # ---- parity spot check against the oracle (rows of the CPU sample + heavy rows)

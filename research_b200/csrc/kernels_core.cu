@@ -135,7 +135,12 @@ __device__ __forceinline__ uint32_t spread_index(uint32_t idx, uint32_t count, u
 // 16 entries 946 -> 553 us, 32 entries 951 -> 942 us).
 // `limit` bounds the lane slots of such a row (narrow_slots; see narrow_limit).
 constexpr uint32_t kNarrowSym = 4096;  // columns of a symbolic row
-constexpr uint32_t kNarrowNum = 1088;  // columns of a numeric row: 9.6 KB a warp, 20 warps per SM
+// Columns of a numeric row: 9.6 KB a warp, 20 warps per SM. The line is not where
+// the occupancy would end it: 1248 slots leave the same 20 warps. 100000 banded
+// rows of 64 entries, whole multiply, at 1088 and at 1248 slots: 1073 columns
+// 1762 and 1767 us, 1201 columns 2873 (in blocks) and 1799 us, 1601 columns 2875
+// and 2864 us (in blocks).
+constexpr uint32_t kNarrowNum = 1088;
 // Lane slots of a row in the steps of one warp: its products, and half a step
 // lost per A entry.
 __host__ __device__ __forceinline__ uint64_t narrow_slots(uint64_t p, uint64_t anz) { return p + 16 * anz; }
@@ -1277,9 +1282,10 @@ __device__ __forceinline__ void mark_bit(unsigned long long* bits, uint32_t c, b
 // slots (one per column) takes the place of an atomic, and there is no block
 // barrier and no owner search. Four entries' loads are in flight. 2 * 10^5
 // banded rows (256/64, 7.2 * 10^8 products), one B200, block kernels -> these:
-// symbolic 1.9 -> 0.8 ms, numeric 4.4 -> 2.2 ms (330 G products/s; 20 warps
-// per SM by the slots, so the loads' latency is what is left); dense blocks
-// 256/64 of 57 entries a row, numeric 1.88 -> 1.3 ms.
+// symbolic 1.9 -> 0.7 ms (held by its instructions: 77% of the issue slots),
+// numeric 4.4 -> 2.2 ms (330 G products/s, held by L1 at 90%: two loads of B, a
+// load and two stores of slot and flag per product; 20 warps per SM by the
+// slots); dense blocks 256/64 of 57 entries a row, numeric 1.88 -> 1.3 ms.
 // op(column offset, value, same) for the products of A entries [a0, a1), by the
 // warp, step by step with a __syncwarp between; `same`: two lanes of the step
 // hold the same column (a B row that repeats one).
@@ -1593,13 +1599,15 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 16 : NT == 256 ? 5 : 1) k_sym_
 //    is the rank of its column, two popcounts away.
 // Rows wider than 2^20 columns are left to k_num_hash. Against the hash table
 // with a radix sort that these rows took before (class kernel, one B200): 2^18
-// uniform rows of 32, bucket form, 13.1 -> 5.2 ms (3.2 GB of C; the gather of
-// the products is 2.0 ms of it, ordering them 1.9 ms, writing them 1.3 ms); 2 * 10^5
-// banded rows (256/64), dense form, 8.0 -> 4.4 ms (165 G products/s, bound by
-// the instructions of the enumeration and of the FP64 shared-memory sums); the
+// uniform rows of 32, bucket form, 13.1 -> 5.4 ms (3.2 GB of C; the gather of
+// the products is 2.0 ms of it, ordering them 1.9 ms, writing them 1.3 ms: the
+// warps wait for the gathers' chain of loads first, 8.1 of 18 cycles between two
+// instructions, then at the row's barriers, 3.5); 2 * 10^5 banded rows (256/64),
+// dense form, 8.0 -> 4.4 ms (165 G products/s; such rows now run a warp each); the
 // power-law 2^17 graph's rows of 512-2048 outputs 0.38 -> 0.20 ms. 64 registers
-// and 32 warps per SM; at 80 registers and 24 warps the bucket form is 10%
-// faster and the dense form 10% slower.
+// and 32 warps per SM; at 80 registers and 24 warps the bucket form was 10%
+// faster and the dense form 10% slower, when the dense form still had the
+// narrow rows.
 constexpr uint32_t kBucketMax = 16;
 template <int NT, int SLOTS>
 struct NumRankSmem {
@@ -2772,6 +2780,9 @@ __global__ void __launch_bounds__(kBitmapThreads, 1)
 //    others are done: 1/32 of the rows of the power-law 2^20 graph times the
 //    graph, 13.3 -> 8.6 ms.
 // All rows of the 2^20 graph as items: 255 ms against 217 ms in k_num_bitmap.
+// The line at kItemWideWords, both sides (class, whole -> items): power-law 2^18
+// graph of 8 entries a row 12.0 -> 10.0 ms, of 16 28.8 -> 27.9; 2^19 columns, whole
+// graph of 8 entries 29.9 -> 24.2, of 16 73.1 -> 74.6, 1/32 of its rows 2.9 -> 2.4.
 constexpr int kItemV = 10240;      // output entries per item (FP64 slots and columns in shared memory)
 constexpr int kItemGroups = 256;   // groups of 32 words (2048 columns) per item
 constexpr int kItemWords = kItemGroups * 32;

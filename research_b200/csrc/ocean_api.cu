@@ -846,11 +846,11 @@ enum Workflow { WF_PRECISE = 0, WF_ESTIMATION = 1, WF_ULTRASPARSE = 2, WF_FAT = 
 //  * estimation when products / nnz(A) reaches estimation_input_expansion_threshold
 //    and the HLL-sampled compaction (products per estimated output) reaches
 //    estimation_output_compaction_threshold twice (sum ratio and mean ratio);
-//  * precise otherwise, for small inputs (no read-back), or when the temporary
+//  * precise otherwise, for small inputs (small_problem_nnz), or when the temporary
 //    output of an estimated workflow would not fit in memory.
 // For the estimation workflow the HLL estimates are left in w.est.
 template <typename RP>
-int choose_workflow(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool readback) {
+int choose_workflow(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStream_t s, bool large) {
   const Config& c = h->cfg;
   // short, fat A times tall, skinny B with few output columns
   // (kernels/SpGEMM.cuh:456-466): every row gets its exact upper bound
@@ -862,9 +862,9 @@ int choose_workflow(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStr
     h->st.estimator = 3;
     return WF_FAT;
   }
-  if (c.force_workflow == WF_PRECISE || (!readback && c.force_workflow < 0)) return WF_PRECISE;
+  if (c.force_workflow == WF_PRECISE || (!large && c.force_workflow < 0)) return WF_PRECISE;
   const DevCounters& k = *h->h_ctr;
-  const uint64_t products = readback ? k.total_products : 0;
+  const uint64_t products = large ? k.total_products : 0;
   if (c.force_workflow == WF_ULTRASPARSE ||
       (c.force_workflow < 0 && c.use_ultrasparse_workflow && A.rows &&
        (double)products / (double)A.rows <= c.usparse_avg_product_threshold &&
@@ -881,7 +881,7 @@ int choose_workflow(ocean_handle* h, const Csr<RP>& A, const Csr<RP>& B, cudaStr
   const bool learned = c.use_learned_estimator;
   if (learned) load_model(h);
   const int log2p = learned ? kLearnedLog2p
-                            : (readback && ratio >= (uint64_t)c.hll_higher_precision_expansion_threshold) ? 6 : 5;
+                            : (large && ratio >= (uint64_t)c.hll_higher_precision_expansion_threshold) ? 6 : 5;
   const double expansion = (log2p == 5 ? 2.0 : 1.5) * c.estimate_scale;
   int samples = (int)(A.rows * c.hll_sample_rate);
   samples = std::max(samples, c.hll_sample_min_rows);
@@ -1058,7 +1058,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
   CResult* owner = new CResult{0};
   try {
     if (A.rows > 0) {
-      const bool readback = run_analysis(h, A, B, s);
+      const bool large = run_analysis(h, A, B, s);
       mark("analysis");
       if (h->cfg.use_segmented_workflow || h->cfg.use_segment_dispatch) {
         // spy-plot segmentation; its records go to the stats (reference:
@@ -1076,7 +1076,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
           mark("segment_dispatch");
         }
       }
-      wf = choose_workflow(h, A, B, s, readback);
+      wf = choose_workflow(h, A, B, s, large);
       mark("workflow");
       // numeric class sizes on the host (grids capped by class size); without
       // them every class is launched at full grid
@@ -1089,14 +1089,14 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
                                 (cf.force_workflow < 0 && cf.use_ultrasparse_workflow));
       const DevCounters& kc = *h->h_ctr;
       const bool fits = kc.max_products <= kUspMaxProducts && kc.total_products < (1ull << 32);
-      if (fits && fusable_cfg && wf == WF_PRECISE && !readback && cf.force_workflow < 0 &&
+      if (fits && fusable_cfg && wf == WF_PRECISE && !large && cf.force_workflow < 0 &&
           (double)kc.total_products <= cf.usparse_avg_product_threshold * (double)A.rows)
         wf = WF_ULTRASPARSE;
       st.fused = fits && fusable_cfg && wf == WF_ULTRASPARSE;
       if (st.fused) {
         nnz = h->h_ctr->total_products;  // C's capacity until the kernel has counted
         st.total_est = nnz;
-      } else if (wf == WF_ULTRASPARSE && readback) {
+      } else if (wf == WF_ULTRASPARSE && large) {
         // the estimates are the product counts, whose total the analysis read
         // back and choose_workflow checked against free memory: no read-back
         st.launches += launch_scan(h->w, h->w.est, h->w.est_off, nullptr, &h->w.ctr->total_est, true, np, s,
@@ -1119,7 +1119,7 @@ void run_spgemm(ocean_handle* h, const ocean_csr_view* Av, const ocean_csr_view*
       // row chunks of equal products (the scan splits the class lists by
       // chunk) so that each chunk's copy to the host overlaps the next ones
       h->w.chunks = 0;
-      if (h->sink_active && wf == WF_PRECISE && readback && !st.fused && !cf.numeric_windows && !track &&
+      if (h->sink_active && wf == WF_PRECISE && large && !st.fused && !cf.numeric_windows && !track &&
           cf.host_pipeline_chunks > 1 && (double)h->h_ctr->total_products >= cf.host_pipeline_min_products) {
         const int k = std::min(cf.host_pipeline_chunks, kMaxChunks);
         const size_t words = (kMaxChunks + 1) + 2 * NB_COUNT * kMaxChunks;
